@@ -118,6 +118,26 @@ __device__ __forceinline__ float far_field_ratio(float4 cm, float3 q) {
   return rdiv(rsqrt_ieee(dot_exact<DIM>(dx, dy, dz, dx, dy, dz)), cm.w);
 }
 
+// farFieldRatio(q) >= beta, decided without the square root and the division
+// where the answer cannot depend on how they round: |q - c|^2 against
+// (beta * diameter)^2.  Forming that threshold costs four roundings (below
+// 2.4e-7 relative) and rounding the root and the quotient moves the reference's
+// ratio by at most 1.2e-7, so outside a band of 2e-6 around the threshold the
+// comparison of the squares gives the reference's answer; inside it (about one
+// test in 10^5) and for thresholds whose square leaves the FP32 normal range
+// the reference's own operations decide.
+template <int DIM>
+__device__ __forceinline__ bool far_enough(float4 cm, float3 q, float beta) {
+  const float dx = rsub(q.x, cm.x), dy = rsub(q.y, cm.y), dz = DIM == 3 ? rsub(q.z, cm.z) : 0.f;
+  const float d2 = dot_exact<DIM>(dx, dy, dz, dx, dy, dz);
+  const float t = rmul(beta, cm.w), t2 = rmul(t, t);
+  if (t > 1e-15f && t < 1e15f && beta > 1e-15f) {
+    if (d2 > rmul(t2, 1.000002f)) return true;
+    if (d2 < rmul(t2, 0.999998f)) return false;
+  }
+  return rdiv(rsqrt_ieee(d2), cm.w) >= beta;
+}
+
 // (int)v as the reference's x86 build evaluates it: NaN/out of range -> INT_MIN.
 __device__ __forceinline__ int trunc_to_int_x86(float v) {
   return (v >= -2147483648.0f && v < 2147483648.0f) ? __float2int_rz(v) : (int)0x80000000;

@@ -106,7 +106,7 @@ __device__ __forceinline__ void bh_warp_task(const DevTree& t, const float* __re
     if (leaf) {
       acc = in && (__int_as_float(0x7f800000) >= beta);
     } else if (in) {
-      acc = far_field_ratio<DIM>(cm, q) >= beta;
+      acc = far_enough<DIM>(cm, q, beta);
     }
     if (VOTE) {
       const unsigned rej = __ballot_sync(0xffffffffu, in && !acc);
