@@ -44,6 +44,22 @@ __global__ void __launch_bounds__(AD_THREADS)
                                 grads);
 }
 
+// A warp per query (bh_query_task): calls of up to bh_query_per_warp() queries.
+template <int DIM, int K, class A>
+__global__ void __launch_bounds__(AD_THREADS)
+    bh_grad_query_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,
+                         const int* __restrict__ order, float beta, KParams kp,
+                         float* __restrict__ out, float* __restrict__ grads,
+                         int* __restrict__ contribs, int* status) {
+  extern __shared__ float4 s_query[];
+  const int warp = threadIdx.x >> 5;
+  const long long slot = (long long)blockIdx.x * AD_WARPS + warp;
+  if (slot >= nq) return;
+  char* scratch = reinterpret_cast<char*>(s_query) + warp * bh_query_smem(t.depth);
+  bh_query_task<DIM, K, A>(t, qsoa, nq, order ? (long long)__ldg(order + slot) : slot, beta, kp,
+                           out, contribs, status, scratch, nullptr, grads);
+}
+
 // --------------------------------------------------------------- sampler ---
 
 template <int DIM, int K, class A>
@@ -155,6 +171,18 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
     const long long blocks = (nq + AD_THREADS - 1) / AD_THREADS;
     bf_grad_kernel<DIM, K, A><<<(unsigned)blocks, AD_THREADS, 0, stream>>>(t, q, nq, kp, out,
                                                                            grads, contribs);
+    return cudaGetLastError();
+  }
+  if (method == SBH_METHOD_BARNES_HUT && bh_query_per_warp(nq, sm_count)) {
+    const size_t smem = AD_WARPS * bh_query_smem(t.depth);
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(bh_grad_query_kernel<DIM, K, A>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    const long long blocks = (nq + AD_WARPS - 1) / AD_WARPS;
+    bh_grad_query_kernel<DIM, K, A><<<(unsigned)blocks, AD_THREADS, smem, stream>>>(
+        t, q, nq, order, beta, kp, out, grads, contribs, status);
     return cudaGetLastError();
   }
   if (method == SBH_METHOD_BARNES_HUT || method == SBH_METHOD_BARNES_HUT_VOTE) {

@@ -9,6 +9,10 @@
 // reference CPU's bit for bit.  With `vote` the lanes accept a node only if all
 // of them do, the reference GPU kernel's __all_sync semantics.
 //
+// Calls of up to bh_query_per_warp() queries take a warp per query instead, its
+// lanes over the next nodes of that query's walk (bh_query_task), with the same
+// results.
+//
 // Node records are read as warp-broadcast loads of 16-byte SoA entries; query
 // order comes from the Morton bucketing in query_sort.cu so the 32 lanes of a
 // warp share most of their walk.
@@ -49,11 +53,28 @@ __global__ void __launch_bounds__(BH_THREADS)
                                                   nullptr, stage);
 }
 
+// A warp per query (bh_query_task).  What bounds it is a step's chain of load,
+// test and compaction; 46-48 registers give 40 warps per SM to hide it.
+template <int DIM, int K>
+__global__ void __launch_bounds__(BH_THREADS)
+    barnes_hut_query_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,
+                            const int* __restrict__ order, float beta, KParams kp,
+                            float* __restrict__ out, int* __restrict__ contribs, int* status) {
+  extern __shared__ float4 s_bh[];
+  const int warp = threadIdx.x >> 5;
+  const long long slot = (long long)blockIdx.x * BH_WARPS + warp;
+  if (slot >= nq) return;
+  char* scratch = reinterpret_cast<char*>(s_bh) + warp * bh_query_smem(t.depth);
+  bh_query_task<DIM, K>(t, qsoa, nq, order ? (long long)__ldg(order + slot) : slot, beta, kp, out,
+                        contribs, status, scratch, nullptr);
+}
+
 // Queries per warp.  A warp's walk covers the union of its lanes' opened sets
 // and each step waits on a node load, so the kernel is latency-bound; when the
 // query count cannot give every SM about 48 warps of 32 queries, warps take
-// fewer queries (down to 4) to have more walks in flight.  Per-query results
-// do not depend on the grouping.  Vote mode keeps 32: its acceptance is defined
+// fewer queries (down to 4) to have more walks in flight (calls that stage leaves;
+// others of that size run a warp per query).  Per-query results do not depend on
+// the grouping.  Vote mode keeps 32: its acceptance is defined
 // over 32 consecutive queries.
 int queries_per_warp(long long nq, bool vote, int sm_count) {
   if (vote) return 32;
@@ -61,6 +82,22 @@ int queries_per_warp(long long nq, bool vote, int sm_count) {
   int g = 32;
   while (g > 4 && (nq + g - 1) / g < want) g /= 2;
   return g;
+}
+
+template <int DIM, int K>
+cudaError_t launch_bh_query(const DevTree& t, const float* q, long long nq, const int* order,
+                            float beta, const KParams& kp, float* out, int* contribs, int* status,
+                            cudaStream_t stream) {
+  const size_t smem = BH_WARPS * bh_query_smem(t.depth);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(barnes_hut_query_kernel<DIM, K>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const long long blocks = (nq + BH_WARPS - 1) / BH_WARPS;
+  barnes_hut_query_kernel<DIM, K><<<(unsigned)blocks, BH_THREADS, smem, stream>>>(
+      t, q, nq, order, beta, kp, out, contribs, status);
+  return cudaGetLastError();
 }
 
 template <int DIM, int K, bool VOTE, bool STAGE>
@@ -91,7 +128,9 @@ cudaError_t launch_barnes_hut(const DevTree& t, int kernel, bool vote, const flo
   if (nq <= 0) return cudaSuccess;
 #define SBH_BH_CASE(D, K)                                                                      \
   if (t.dim == D && kernel == K)                                                               \
-    return vote           ? launch_bh<D, K, true, false>(t, q, nq, order, beta, kp, out,       \
+    return !vote && !stage_leaves && bh_query_per_warp(nq, sm_count)                           \
+               ? launch_bh_query<D, K>(t, q, nq, order, beta, kp, out, contribs, status, stream) \
+           : vote         ? launch_bh<D, K, true, false>(t, q, nq, order, beta, kp, out,       \
                                                          contribs, status, stream, sm_count)   \
            : stage_leaves ? launch_bh<D, K, false, true>(t, q, nq, order, beta, kp, out,       \
                                                          contribs, status, stream, sm_count)   \

@@ -31,6 +31,13 @@ bool wants_sort(const sbh_params* p) {
   return p->method == SBH_METHOD_BARNES_HUT || p->method == SBH_METHOD_STOCHASTIC;
 }
 
+// Whether a call of nq queries is worth ordering (small Barnes-Hut calls are not).
+bool needs_order(const sbh_gpu_tree* tree, const sbh_params* p, int64_t nq) {
+  if (!wants_sort(p)) return false;
+  return !(p->method == SBH_METHOD_BARNES_HUT && !(p->flags & SBH_FLAG_STAGE_LEAVES) &&
+           nq <= sbh::kBhUnorderedQueries && sbh::bh_query_per_warp(nq, tree->sm_count));
+}
+
 // Enqueues one evaluation.  With `grad` the adjoint kernels run instead (values
 // and, when d_grads is non-null, gradients).
 cudaError_t run_eval(sbh_gpu_tree* tree, const sbh_params* p, const float* d_q, int64_t nq,
@@ -41,7 +48,7 @@ cudaError_t run_eval(sbh_gpu_tree* tree, const sbh_params* p, const float* d_q, 
   kp.alpha = std::isnan(p->alpha) ? t.alpha : p->alpha;
   kp.eps2 = p->eps * p->eps;
   const int* order = nullptr;
-  if (wants_sort(p) && nq > 0) {
+  if (needs_order(tree, p, nq) && nq > 0) {
     cudaError_t e = sbh::launch_query_sort(d_q, nq, t.dim, d_sortws, d_order, stream);
     if (e != cudaSuccess) return e;
     order = d_order;
@@ -193,7 +200,7 @@ int device_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* d_que
   void* tmp = nullptr;
   int* d_ord = nullptr;
   void* d_sort = nullptr;
-  if (wants_sort(params)) {
+  if (needs_order(tree, params, nq)) {
     const size_t b_ord = align256((size_t)nq * sizeof(int));
     cudaMemPool_t pool = nullptr;
     st = scratch_pool(tree->device, &pool);

@@ -10,6 +10,20 @@ namespace sbh {
 cudaError_t launch_brute_force(const DevTree& t, int kernel, const float* q, long long nq,
                                const KParams& kp, float* out, cudaStream_t stream, int sm_count);
 
+// Barnes-Hut calls of up to 2,048 queries per SM run a warp per query
+// (bh_query_task), larger ones a lane per query (bh_warp_task).  A lane per query
+// does a node test in fewer instructions, but a call lasts at least as long as
+// its longest walk, one node after the other.  Measured on B200 (us, lane / warp
+// per query, theta 0.5): 1M-point torus, branching 64: 1,000 queries 3,482 / 205,
+// 65,536 5,054 / 1,015, 200,000 6,179 / 2,741, 1M 10,269 / 13,348; 10,000-point
+// Gaussian mixture, branching 8: 648 / 80, 810 / 227, 894 / 549, 1,315 / 2,550.
+inline bool bh_query_per_warp(long long nq, int sm_count) { return nq <= 2048LL * sm_count; }
+// Without neighbours sharing a warp the query order only helps the L1 cache; up
+// to this many queries that is worth less than the ordering's seven launches
+// (16,000 queries on the same trees: 379 -> 384 and 122 -> 94 us without it;
+// 65,536: 1,015 -> 1,105 and 227 -> 220).
+constexpr long long kBhUnorderedQueries = 16384;
+
 // stage_leaves: accepted multi-point leaves are copied to shared memory by bulk
 // asynchronous copies (SBH_FLAG_STAGE_LEAVES; not with vote).
 cudaError_t launch_barnes_hut(const DevTree& t, int kernel, bool vote, const float* q,

@@ -21,7 +21,11 @@
 // float, div by a float, warp shuffles of a value (shfl, shfl_up), point() and
 // node() (the value of one source record or
 // node aggregate at query q), and store() (writes the result and, when the
-// caller asks, the gradient as structure-of-arrays [dim][nq]).
+// caller asks, the gradient as structure-of-arrays [dim][nq]).  For sums whose
+// terms are evaluated by several lanes: kOrdered says that ordered(), the part of
+// a value whose additions must happen in the reference's order, exists; add_rest()
+// adds the other parts, which lanes may group as they like, and join() puts an
+// ordered sum and the rest together.
 #pragma once
 
 #include "device_common.cuh"
@@ -62,6 +66,10 @@ template <int DIM, int K>
 struct SumF {
   using V = float;
   static constexpr bool kGrad = false;
+  static constexpr bool kOrdered = true;
+  __device__ __forceinline__ static float ordered(V a) { return a; }
+  __device__ __forceinline__ static V add_rest(V a, V) { return a; }
+  __device__ __forceinline__ static V join(float sum, V) { return sum; }
   __device__ __forceinline__ static V zero() { return 0.f; }
   __device__ __forceinline__ static V nan() { return __int_as_float(0x7fc00000); }
   __device__ __forceinline__ static V add(V a, V b) { return radd(a, b); }
@@ -97,6 +105,14 @@ struct SumGrad {
   static_assert(K == kGravity || K == kPlummer, "gradients of gravity and Plummer only");
   using V = GradValue;
   static constexpr bool kGrad = true;
+  static constexpr bool kOrdered = true;
+  __device__ __forceinline__ static float ordered(V a) { return a.v; }
+  __device__ __forceinline__ static V add_rest(V a, V b) {
+    return V{a.v, a.gx + b.gx, a.gy + b.gy, a.gz + b.gz};
+  }
+  __device__ __forceinline__ static V join(float sum, V rest) {
+    return V{sum, rest.gx, rest.gy, rest.gz};
+  }
   __device__ __forceinline__ static V zero() { return V{0.f, 0.f, 0.f, 0.f}; }
   __device__ __forceinline__ static V nan() {
     const float n = __int_as_float(0x7fc00000);
@@ -163,6 +179,10 @@ template <int DIM>
 struct SumLse {
   using V = LseValue;
   static constexpr bool kGrad = true;
+  static constexpr bool kOrdered = false;
+  __device__ __forceinline__ static float ordered(V) { return 0.f; }
+  __device__ __forceinline__ static V add_rest(V a, V b) { return add(a, b); }
+  __device__ __forceinline__ static V join(float, V rest) { return rest; }
   __device__ __forceinline__ static V zero() {
     return V{-__int_as_float(0x7f800000), 0.f, 0.f, 0.f, 0.f};
   }

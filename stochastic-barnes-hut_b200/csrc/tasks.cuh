@@ -169,6 +169,185 @@ __device__ __forceinline__ void bh_warp_task(const DevTree& t, const float* __re
   }
 }
 
+// ---- one query, a warp's lanes over the nodes of its walk --------------------
+
+// Warp scratch of bh_query_task: the stack, then 64 terms waiting to be added
+// and the 32 window positions' owners.
+struct BhEntry {
+  int a;  // first node or point; a term's value (float bits)
+  int b;  // > 0: nodes [a, a + b); < 0: points [a, a - b); 0: a term
+};
+constexpr int kBhQueryEntries = 160;  // besides one entry per tree level
+__host__ __device__ constexpr int bh_query_entries(int depth) { return kBhQueryEntries + depth; }
+__host__ __device__ constexpr size_t bh_query_smem(int depth) {
+  return ((size_t)bh_query_entries(depth) * sizeof(BhEntry) + 15) / 16 * 16 + 64 * 4 + 32 * 4;
+}
+
+// One warp evaluates one query.  bh_warp_task above gives each lane a query and
+// pays one load latency and one step per node of the union of the lanes' walks;
+// with few queries that serial chain is all the time there is.  Here the lanes
+// are the next 32 nodes (or leaf points) of one query's walk.
+//
+// The walk's state is the rest of the depth-first sequence, first entry on top
+// of a stack: ranges of sibling nodes not yet tested, ranges of points of
+// accepted leaves, and terms already evaluated that wait for the ranges before
+// them.  A step takes the entries on top that hold the next 32 nodes and points,
+// one each per lane: tests a node (far_enough), evaluates an accepted node or a
+// point, and puts the outcomes back in place -- an accepted node becomes its
+// term, an opened one the range of its children, an accepted leaf of several
+// points the range of its points.  The terms before the first range are then
+// the next ones of the depth-first sequence and are added one after the other.
+// So exactly evaluateBarnesHut_stackless's nodes are opened and its terms are
+// added in its order (include/barnes_hut.h:23-78): bit-identical results.  Parts
+// of a value that need no order (gradients, the smooth distance's max-shifted
+// sum) are added lane by lane and joined at the end.
+//
+// A step nets at most as many new entries as it takes nodes; when the room left
+// (less one entry per level) is below 32 it takes fewer, down to one, which is
+// the plain depth-first walk, so the stack cannot overflow.
+template <int DIM, int K, class A = SumF<DIM, K>>
+__device__ __forceinline__ void bh_query_task(const DevTree& t, const float* __restrict__ qsoa,
+                                              long long nq, long long qi, float beta,
+                                              const KParams& kp, float* __restrict__ out,
+                                              int* __restrict__ contribs, int* status,
+                                              char* scratch,
+                                              const float* __restrict__ self_mass,
+                                              float* __restrict__ grads = nullptr) {
+  using V = typename A::V;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int cap = bh_query_entries(t.depth);
+  BhEntry* stk = reinterpret_cast<BhEntry*>(scratch);
+  float* seq = reinterpret_cast<float*>(scratch + ((size_t)cap * sizeof(BhEntry) + 15) / 16 * 16);
+  int* owner_of = reinterpret_cast<int*>(seq + 64);
+  const float3 q = load_query<DIM>(qsoa, nq, qi);
+  float total = 0.f;
+  V rest = A::zero();
+  int nc = 0;
+  if (lane == 0) stk[0] = BhEntry{0, 1};
+  __syncwarp();
+  int sp = 1;
+  long long budget = 2 * (t.nn + t.n) + 2;  // a step takes a node, a point or a term, each once
+  while (sp > 0) {
+    if (--budget < 0) {
+      if (lane == 0) report_status(status, kStatusTraversalLimit);
+      break;
+    }
+    const int room = cap - t.depth - 2 - sp;
+    const int window = room >= 32 ? 32 : max(room, 1);
+    // Entry lanes: lane l looks at the l-th entry from the top.
+    BhEntry e = lane < sp ? stk[sp - 1 - lane] : BhEntry{0, 0};
+    const bool have = lane < sp;
+    const int cnt = min(abs(e.b), 64);  // beyond the window all the same
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(full, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int excl = incl - cnt;
+    const bool used = have && excl < window;
+    const unsigned used_mask = __ballot_sync(full, used);
+    const unsigned term_mask = __ballot_sync(full, used && cnt == 0);
+    const int n_used = __popc(used_mask);  // used entries are the first n_used lanes
+    const int taken = min(__shfl_sync(full, incl, n_used - 1), window);
+    if (used && cnt > 0) owner_of[excl] = lane;
+    const unsigned starts = __reduce_or_sync(full, used && cnt > 0 ? 1u << excl : 0u);
+    __syncwarp();
+    // Node lanes: lane l takes the l-th node or point of the window.
+    const bool item = lane < taken;
+    const int head = 31 - __clz(starts & (below | (1u << lane)));
+    const int owner = owner_of[item ? head : 0] & 31;
+    const int ea = __shfl_sync(full, e.a, owner), eb = __shfl_sync(full, e.b, owner);
+    const int idx = ea + lane - head;
+    bool is_term = false, is_range = false;
+    float val = 0.f;
+    BhEntry r = BhEntry{0, 0};
+    if (item) {
+      if (eb > 0) {
+        const int4 topo = __ldg(t.nd_topo + idx);
+        const float4 cm = __ldg(t.nd_cm + idx);
+        const float4 ag = __ldg(t.nd_agg + idx);
+        const bool leaf = topo.y == 0;
+        const bool acc = leaf ? __int_as_float(0x7f800000) >= beta : far_enough<DIM>(cm, q, beta);
+        if (!acc) {
+          is_range = !leaf;
+          r = BhEntry{topo.x, topo.y};
+        } else if (leaf && topo.w - topo.z != 1) {
+          is_range = topo.w > topo.z;
+          r = BhEntry{topo.z, topo.z - topo.w};
+        } else {
+          const V v = A::node(cm, ag, q, kp);
+          is_term = A::kOrdered;
+          val = A::ordered(v);
+          rest = A::add_rest(rest, v);
+          nc++;
+        }
+      } else {
+        const V v = A::point(__ldg(t.pt_pm + idx), __ldg(t.pt_nrm + idx), q, kp);
+        is_term = A::kOrdered;
+        val = A::ordered(v);
+        rest = A::add_rest(rest, v);
+        nc++;
+      }
+    }
+    // The window's outcomes in depth-first order: position of a node lane's own,
+    // and of a waiting term's.
+    const unsigned outs = __ballot_sync(full, is_term || is_range);
+    const unsigned ranges = __ballot_sync(full, is_range);
+    const int pos = __popc(outs & below) + __popc(term_mask & ((1u << owner) - 1u));
+    const unsigned before_e = excl >= 32 ? full : (1u << excl) - 1u;
+    const int epos = __popc(term_mask & below) + __popc(outs & before_e);
+    const int n_out = __popc(outs) + __popc(term_mask);
+    const int first = ranges ? __shfl_sync(full, pos, __ffs(ranges) - 1) : n_out;
+    // A range the window covers only in part stays below the outcomes.
+    const bool cut = used && incl > window;
+    int base = sp - n_used;
+    if (cut) {
+      const int k = window - excl;
+      stk[base] = e.b > 0 ? BhEntry{e.a + k, e.b - k} : BhEntry{e.a + k, e.b + k};
+    }
+    if (__any_sync(full, cut)) base++;
+    const int top = base + n_out - first - 1;  // index of the outcome at position `first`
+    if (is_term || is_range) {
+      if (pos < first)
+        seq[pos] = val;
+      else
+        stk[top - (pos - first)] = is_range ? r : BhEntry{__float_as_int(val), 0};
+    }
+    if (used && cnt == 0) {
+      if (epos < first)
+        seq[epos] = __int_as_float(e.a);
+      else
+        stk[top - (epos - first)] = e;
+    }
+    __syncwarp();
+    sp = top + 1;
+    if (A::kOrdered) {
+      int k = 0;
+      for (; k + 4 <= first; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(seq + k);
+        total = radd(radd(radd(radd(total, x.x), x.y), x.z), x.w);
+      }
+      for (; k < first; k++) total = radd(total, seq[k]);
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nc += __shfl_xor_sync(full, nc, o);
+    if (A::kGrad) rest = A::add_rest(rest, A::shfl(rest, lane ^ o));
+  }
+  if (lane == 0) {
+    V v = A::join(total, rest);
+    if (self_mass) v = A::sub(v, self_term<DIM, K, A>(q, __ldg(self_mass + qi), kp));
+    A::store(out, grads, nq, qi, v, kp);
+    if (contribs) contribs[qi] = nc;
+  }
+  __syncwarp();
+}
+
 // ============================================================ sampler ===
 
 // acc += k(point) for every point of leaf tc, in order (rare: leaves with
