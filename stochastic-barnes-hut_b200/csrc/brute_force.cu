@@ -2,198 +2,121 @@
 // include/brute_force_gpu.h:18-66, and its wrappers src/sbh_gpu.cu:39-77).
 //
 // Design (B200):
-//   * A cluster of C CTAs owns one tile of THREADS*BF_QPT queries; CTA rank r
-//     sums source chunk r of C.  The C partial sums of a query are combined in
-//     rank order through distributed shared memory, so there is no global
-//     scratch buffer and no second launch, and results are deterministic.
-//   * Each thread carries BF_QPT = 8 queries as four pairs, and the pairwise
-//     arithmetic runs on Blackwell's packed FP32 instructions (FADD2 / FMUL2 /
-//     FFMA2, two lanes of FP32 per issue): a Plummer pair costs 3.5 FP32 issue
-//     slots plus one MUFU rsqrt, so the kernel is bound by the MUFU pipe (16
-//     results per clock per SM), not by issue.
-//   * Sources are staged in shared memory with every coordinate duplicated into
-//     both halves of a float2 (x,x | y,y | z,z | m,m), so one broadcast
-//     shared load gives the packed operand directly.
-//   * Compensated accumulation in two levels: plain FP32 over BF_SUB sources,
-//     then a Knuth two-sum into a (sum, error) pair -- the reference's Kahan
-//     loop (brute_force_gpu.h:52-60) at ~1/BF_SUB of its cost per pair.
-//   * Grid shape: the launcher picks the CTA size (64 or 128 threads) and the
-//     cluster size (1-8) that spread the CTAs most evenly over the SMs.
-#include <cooperative_groups.h>
-
+//   * A warp carries 8 queries (2 in calls of few) and its lanes split the sources;
+//     warps of a CTA and CTAs of a cluster split them further as the call's shape
+//     asks (split_sum.cuh).  With a query per thread instead -- the sources
+//     staged in shared memory -- a call of up to 4,000 queries filled 16 of the
+//     148 SMs with two warps each: 997 queries x 1,000,003 sources, smooth
+//     distance, took 11,697 us, now 570.
+//   * The queries are packed pairs and the pairwise arithmetic runs on Blackwell's
+//     FP32x2 instructions (FADD2 / FMUL2 / FFMA2, two lanes of FP32 per issue): a
+//     Plummer pair costs 3.5 FP32 issue slots plus one MUFU rsqrt.  Both pipes are
+//     loaded: 65,536 x 65,536 Plummer pairs take 1,180 us (0.79 of the MUFU bound;
+//     1,350 with a query per thread), smooth distance 1,980 (2,322), winding
+//     number 2,348 (2,519), gravity 2,105 (2,309).
+//   * Compensated accumulation in two levels: plain FP32 over 32 sources of a
+//     lane, then a Knuth two-sum into a (sum, error) pair -- the reference's Kahan
+//     loop (brute_force_gpu.h:52-60) at a fraction of its cost per pair.
 #include "launch.h"
 #include "pairs.cuh"
+#include "split_sum.cuh"
 #include "tasks.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace sbh {
 namespace {
 
-constexpr int BF_QPT = 8;                 // queries per thread
-constexpr int BF_PAIRS = BF_QPT / 2;      // packed query pairs per thread
-constexpr int BF_TILE = 512;              // sources per shared-memory stage
-constexpr int BF_SUB = 64;                // sources per plain partial sum
-
-template <int THREADS, int DIM, int K>
-__global__ void __launch_bounds__(THREADS) brute_force_kernel(DevTree t,
-                                                              const float* __restrict__ qsoa,
-                                                              long long nq, KParams kp,
-                                                              float* __restrict__ out) {
-  constexpr bool kNormals = (K == kWindingNumber);
-  constexpr int kQueriesPerCta = THREADS * BF_QPT;
-  __shared__ SrcPair s_src[BF_TILE];
-  __shared__ NrmPair s_nrm[kNormals ? BF_TILE : 1];
-  __shared__ float2 s_part[kQueriesPerCta];
-
-  cg::cluster_group cluster = cg::this_cluster();
-  const int csize = (int)cluster.num_blocks();
-  const int rank = (int)cluster.block_rank();
-  const long long tile = blockIdx.x / csize;
-  const long long q0 = tile * kQueriesPerCta;
-
-  // Query j of this thread is q0 + threadIdx.x + j * THREADS; pair p holds
-  // queries 2p and 2p+1, negated so the differences are packed adds.
-  float2 nqx[BF_PAIRS], nqy[BF_PAIRS], nqz[BF_PAIRS];
-#pragma unroll
-  for (int p = 0; p < BF_PAIRS; p++) {
-    float3 a = make_float3(0.f, 0.f, 0.f), b = a;
-    const long long qa = q0 + threadIdx.x + (2 * p) * THREADS;
-    const long long qb = qa + THREADS;
-    if (qa < nq) a = load_query<DIM>(qsoa, nq, qa);
-    if (qb < nq) b = load_query<DIM>(qsoa, nq, qb);
-    nqx[p] = make_float2(-a.x, -b.x);
-    nqy[p] = make_float2(-a.y, -b.y);
-    nqz[p] = make_float2(-a.z, -b.z);
+// A lane's compensated sum of one query.
+struct PlainSum {
+  float hi, lo;
+  __device__ __forceinline__ void merge(const PlainSum& b) {
+    two_sum_add(hi, lo, b.hi);
+    lo += b.lo;
   }
-  float hi[BF_QPT], lo[BF_QPT];
-#pragma unroll
-  for (int j = 0; j < BF_QPT; j++) hi[j] = lo[j] = 0.f;
+};
 
-  const long long chunk = (t.n + csize - 1) / csize;
-  const long long c0 = min((long long)rank * chunk, t.n);
-  const long long c1 = min(c0 + chunk, t.n);
-  const NrmPair no_normal = {};
-  for (long long base = c0; base < c1; base += BF_TILE) {
-    const int len = (int)min((long long)BF_TILE, c1 - base);
-    for (int k = threadIdx.x; k < len; k += THREADS) {
-      const float4 v = __ldg(t.pt_pm + base + k);
-      s_src[k] = SrcPair{dup(v.x), dup(v.y), dup(v.z), dup(v.w)};
-      if (kNormals) {
-        const float4 n = __ldg(t.pt_nrm + base + k);
-        s_nrm[k] = NrmPair{dup(n.x), dup(n.y), dup(n.z), dup(0.f)};
-      }
-    }
-    __syncthreads();
-    for (int sb = 0; sb < len; sb += BF_SUB) {
-      const int se = min(sb + BF_SUB, len);
-      float2 part[BF_PAIRS];
-#pragma unroll
-      for (int p = 0; p < BF_PAIRS; p++) part[p] = make_float2(0.f, 0.f);
-      if (K == kSmoothDist) {
-        // its exponential split between the MUFU and the FP32 pipe (pairs.cuh)
-        const auto src = [&](int k) { return s_src[sb + k]; };
-        if (se - sb == BF_SUB)
-          accumulate_smooth<DIM, BF_PAIRS, BF_SUB>(part, src, BF_SUB, nqx, nqy, nqz, kp);
-        else
-          accumulate_smooth<DIM, BF_PAIRS, 0>(part, src, se - sb, nqx, nqy, nqz, kp);
-      } else if (se - sb == BF_SUB) {
-#pragma unroll 4
-        for (int k = sb; k < sb + BF_SUB; k++) {
-          const SrcPair sp = s_src[k];
-          const NrmPair np = kNormals ? s_nrm[k] : no_normal;
-#pragma unroll
-          for (int p = 0; p < BF_PAIRS; p++)
-            part[p] = accumulate2<DIM, K>(part[p], sp, np, nqx[p], nqy[p], nqz[p], kp);
-        }
-      } else {
-        for (int k = sb; k < se; k++) {
-          const SrcPair sp = s_src[k];
-          const NrmPair np = kNormals ? s_nrm[k] : no_normal;
-#pragma unroll
-          for (int p = 0; p < BF_PAIRS; p++)
-            part[p] = accumulate2<DIM, K>(part[p], sp, np, nqx[p], nqy[p], nqz[p], kp);
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < BF_PAIRS; p++) {
-        two_sum_add(hi[2 * p], lo[2 * p], part[p].x);
-        two_sum_add(hi[2 * p + 1], lo[2 * p + 1], part[p].y);
-      }
-    }
-    __syncthreads();
-  }
+// A lane's NP query pairs (split_sum.cuh).
+template <int DIM, int K, int NP>
+struct PlainAcc {
+  using Sum = PlainSum;
+  static constexpr int Q = 2 * NP;
+  static constexpr int kMinCtas = NP == 4 ? 2 : K == kWindingNumber ? 3 : 4;  // no spills
+  static constexpr bool kNormals = K == kWindingNumber;
+  float2 nqx[NP], nqy[NP], nqz[NP], part[NP];
+  float hi[Q], lo[Q];
+  KParams kp;
 
+  __device__ __forceinline__ void load(const float* qsoa, long long nq, long long q0,
+                                       const KParams& params) {
+    kp = params;
 #pragma unroll
-  for (int j = 0; j < BF_QPT; j++) s_part[threadIdx.x + j * THREADS] = make_float2(hi[j], lo[j]);
-  cluster.sync();
-  if (rank == 0) {
-    for (int r = 1; r < csize; r++) {
-      const float2* peer = cluster.map_shared_rank(s_part, r);
-#pragma unroll
-      for (int j = 0; j < BF_QPT; j++) {
-        const float2 v = peer[threadIdx.x + j * THREADS];
-        two_sum_add(hi[j], lo[j], v.x);
-        lo[j] += v.y;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < BF_QPT; j++) {
-      const long long qi = q0 + threadIdx.x + j * THREADS;
-      const float v = hi[j] + lo[j];
-      if (qi < nq) out[qi] = K == kGravity ? -v : v;
+    for (int p = 0; p < NP; p++) {
+      float3 a = make_float3(0.f, 0.f, 0.f), b = a;
+      if (q0 + 2 * p < nq) a = load_query<DIM>(qsoa, nq, q0 + 2 * p);
+      if (q0 + 2 * p + 1 < nq) b = load_query<DIM>(qsoa, nq, q0 + 2 * p + 1);
+      nqx[p] = make_float2(-a.x, -b.x);
+      nqy[p] = make_float2(-a.y, -b.y);
+      nqz[p] = make_float2(-a.z, -b.z);
+      part[p] = make_float2(0.f, 0.f);
+      hi[2 * p] = lo[2 * p] = hi[2 * p + 1] = lo[2 * p + 1] = 0.f;
     }
   }
-  // Peers keep their shared memory alive until rank 0 has read it.
-  cluster.sync();
-}
-
-template <int THREADS, int DIM, int K>
-cudaError_t launch_bf_shape(const DevTree& t, const float* q, long long nq, const KParams& kp,
-                            float* out, cudaStream_t stream, int csize) {
-  const long long tiles = (nq + THREADS * BF_QPT - 1) / (THREADS * BF_QPT);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * csize), 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, brute_force_kernel<THREADS, DIM, K>, t, q, nq, kp, out);
-}
+  template <int MODE>
+  __device__ __forceinline__ void add(float4 s, float4 n) {
+    const SrcPair sp = {dup(s.x), dup(s.y), dup(s.z), dup(s.w)};
+    const NrmPair np = {dup(n.x), dup(n.y), dup(n.z), dup(0.f)};
+#pragma unroll
+    for (int p = 0; p < NP; p++)
+      part[p] = accumulate2<DIM, K, MODE>(part[p], sp, np, nqx[p], nqy[p], nqz[p], kp);
+  }
+  __device__ __forceinline__ bool scaled() const { return K == kSmoothDist && kp.alpha >= 0.f; }
+  __device__ __forceinline__ void group(const float4 (&s)[kSplitGroup],
+                                        const float4 (&n)[kSplitGroup]) {
+    static_assert(kSplitGroup == kSdFmaEvery, "one source of a group on the FP32 pipe");
+    if (scaled()) {
+      add<2>(s[0], n[0]);
+#pragma unroll
+      for (int i = 1; i < kSplitGroup; i++) add<1>(s[i], n[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kSplitGroup; i++) add<0>(s[i], n[i]);
+    }
+  }
+  __device__ __forceinline__ void single(float4 s, float4 n) {
+    if (scaled())
+      add<1>(s, n);
+    else
+      add<0>(s, n);
+  }
+  __device__ __forceinline__ void flush() {
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      if (scaled()) part[p] = __fmul2_rn(part[p], dup(kExp2Unscale));
+      two_sum_add(hi[2 * p], lo[2 * p], part[p].x);
+      two_sum_add(hi[2 * p + 1], lo[2 * p + 1], part[p].y);
+      part[p] = make_float2(0.f, 0.f);
+    }
+  }
+  __device__ __forceinline__ Sum sum(int j) const { return Sum{hi[j], lo[j]}; }
+  __device__ __forceinline__ static void store(float* out, float*, long long, long long qi,
+                                               const Sum& s, const KParams&) {
+    const float v = s.hi + s.lo;
+    out[qi] = K == kGravity ? -v : v;
+  }
+};
 
 template <int DIM, int K>
 cudaError_t launch_bf(const DevTree& t, const float* q, long long nq, const KParams& kp, float* out,
                       cudaStream_t stream, int sm_count) {
-  // Every CTA does the same work (THREADS * BF_QPT queries x n / csize
-  // sources) and the kernel is bound per SM, so the run takes about
-  // ceil(CTAs / SMs) CTA-times.  Pick the shape with the least of that time,
-  // preferring fewer clusters (less reduction) on ties; never split sources
-  // below two stages per CTA.
-  int best_threads = 128, best_c = 1;
-  double best = -1.0;
-  for (int threads : {128, 64}) {
-    const long long tiles = (nq + threads * BF_QPT - 1) / (threads * BF_QPT);
-    for (int c = 1; c <= 8; c *= 2) {
-      if (c > 1 && t.n < (long long)BF_TILE * c * 2) break;
-      const long long ctas = tiles * c;
-      const double waves = (double)((ctas + sm_count - 1) / sm_count);
-      const double cost = waves * threads / c;
-      if (best < 0.0 || cost < best * 0.999) {
-        best = cost;
-        best_threads = threads;
-        best_c = c;
-      }
-    }
-  }
-  if (best_threads == 128)
-    return launch_bf_shape<128, DIM, K>(t, q, nq, kp, out, stream, best_c);
-  return launch_bf_shape<64, DIM, K>(t, q, nq, kp, out, stream, best_c);
+  // 8 queries a warp, or 2 where that spreads a call of few over more warps: per
+  // source a warp of 2 takes 0.55 of the time of one of 8.  Measured (us, 8 / 2 a
+  // warp, smooth distance, 1M sources): 1 query 65 / 40, 40 67 / 52, 200 151 / 156.
+  using Eight = PlainAcc<DIM, K, 4>;
+  using Two = PlainAcc<DIM, K, 1>;
+  const SplitShape s8 = split_shape(nq, t.n, Eight::Q, Eight::kMinCtas, sm_count);
+  const SplitShape s2 = split_shape(nq, t.n, Two::Q, Two::kMinCtas, sm_count);
+  if (0.55 * s2.cost < s8.cost)
+    return launch_split<Two, DIM>(t, q, nq, kp, out, nullptr, nullptr, stream, s2);
+  return launch_split<Eight, DIM>(t, q, nq, kp, out, nullptr, nullptr, stream, s8);
 }
 
 }  // namespace

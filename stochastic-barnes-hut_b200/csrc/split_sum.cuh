@@ -1,0 +1,187 @@
+// All-pairs sums with the sources split over a warp's lanes (the plain sums,
+// brute_force.cu, and the gradients, adjoint.cu).
+//
+// A warp carries Q queries, the same ones in every lane as packed FP32x2 pairs,
+// and its lanes take every 32nd source of a range, so 1 to 8 queries are enough
+// to keep a warp busy.  What is left of the parallelism goes over the sources:
+// `sw` of a CTA's 8 warps take parts of the sources of the same queries (the
+// others have queries of their own and read the same sources through L1), and a
+// cluster of up to 16 CTAs splits them further.  Every lane sums plain FP32 runs
+// of kSplitRun sources and merges each into a compensated sum; lanes, warps and CTAs
+// (through distributed shared memory, in rank order) merge those.  No scratch
+// memory, one launch, and the result depends only on the call's shape.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "device_common.cuh"
+
+namespace sbh {
+namespace {
+
+constexpr int kSplitWarps = 8;
+constexpr int kSplitThreads = 32 * kSplitWarps;
+constexpr int kSplitGroup = 4;  // sources a lane loads at a time
+constexpr int kSplitRun = 32;   // sources of a plain FP32 sum
+
+template <class T>
+__device__ __forceinline__ T shfl_down_words(const T& v, int d) {
+  static_assert(sizeof(T) % 4 == 0, "word-sized members");
+  T r;
+  const int* src = reinterpret_cast<const int*>(&v);
+  int* dst = reinterpret_cast<int*>(&r);
+#pragma unroll
+  for (int w = 0; w < (int)(sizeof(T) / 4); w++) dst[w] = __shfl_down_sync(0xffffffffu, src[w], d);
+  return r;
+}
+
+// Acc: a lane's state for Q queries.  load() reads them, group() adds
+// kSplitGroup sources, single() one, flush() ends a run, sum(j) is query j's
+// compensated sum (Acc::Sum, with merge()), store() writes a query's result.
+template <class Acc, int DIM>
+__global__ void __launch_bounds__(kSplitThreads, Acc::kMinCtas)
+    split_sum_kernel(DevTree t, const float* __restrict__ qsoa, long long nq, KParams kp, int sw,
+                     float* __restrict__ out, float* __restrict__ grads,
+                     int* __restrict__ contribs) {
+  using Sum = typename Acc::Sum;
+  constexpr int Q = Acc::Q;
+  __shared__ Sum s_warp[kSplitWarps * Q];
+  __shared__ Sum s_cta[kSplitWarps * Q];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int csize = (int)cluster.num_blocks();
+  const int rank = (int)cluster.block_rank();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tiles = kSplitWarps / sw;  // query tiles of this CTA
+  const long long tile0 = (long long)(blockIdx.x / csize) * tiles;
+  const int parts = csize * sw;
+  const long long chunk = ((t.n + parts - 1) / parts + 31) / 32 * 32;
+  const long long c0 = min((long long)(rank * sw + warp % sw) * chunk, t.n);
+  const long long c1 = min(c0 + chunk, t.n);
+
+  Acc acc;
+  acc.load(qsoa, nq, (tile0 + warp / sw) * Q, kp);
+  // The next group is loaded before the current one is summed.
+  const long long full_end = c0 + (c1 - c0) / (32 * kSplitGroup) * (32 * kSplitGroup);
+  long long base = c0;
+  float4 s[kSplitGroup], nr[kSplitGroup], s2[kSplitGroup], nr2[kSplitGroup];
+  auto fetch = [&](long long at, float4 (&s)[kSplitGroup], float4 (&nr)[kSplitGroup]) {
+#pragma unroll
+    for (int i = 0; i < kSplitGroup; i++) {
+      s[i] = __ldg(t.pt_pm + at + 32 * i + lane);
+      nr[i] = Acc::kNormals ? __ldg(t.pt_nrm + at + 32 * i + lane)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (base < full_end) fetch(base, s, nr);
+  int run = 0;
+  for (; base < full_end; base += 32 * kSplitGroup) {
+    const bool more = base + 32 * kSplitGroup < full_end;
+    if (more) fetch(base + 32 * kSplitGroup, s2, nr2);
+    acc.group(s, nr);
+    if ((++run & (kSplitRun / kSplitGroup - 1)) == 0) acc.flush();
+#pragma unroll
+    for (int i = 0; i < kSplitGroup; i++) {
+      s[i] = s2[i];
+      nr[i] = nr2[i];
+    }
+  }
+  for (base += lane; base < c1; base += 32)
+    acc.single(__ldg(t.pt_pm + base), Acc::kNormals ? __ldg(t.pt_nrm + base)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f));
+  acc.flush();
+
+#pragma unroll
+  for (int j = 0; j < Q; j++) {
+    Sum v = acc.sum(j);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v.merge(shfl_down_words(v, o));
+    if (lane == 0) s_warp[warp * Q + j] = v;
+  }
+  __syncthreads();
+  const int mine = threadIdx.x;  // this thread's query of the CTA's, if it has one
+  const bool has = mine < tiles * Q;
+  Sum v;
+  if (has) {
+    v = s_warp[(mine / Q) * sw * Q + mine % Q];
+    for (int p = 1; p < sw; p++) v.merge(s_warp[((mine / Q) * sw + p) * Q + mine % Q]);
+    s_cta[mine] = v;
+  }
+  if (csize > 1) cluster.sync();
+  if (rank == 0 && has) {
+    for (int r = 1; r < csize; r++) v.merge(cluster.map_shared_rank(s_cta, r)[mine]);
+    const long long qi = tile0 * Q + mine;
+    if (qi < nq) {
+      Acc::store(out, grads, nq, qi, v, kp);
+      if (contribs) contribs[qi] = (int)t.n;
+    }
+  }
+  // Peers keep their shared memory alive until rank 0 has read it.
+  if (csize > 1) cluster.sync();
+}
+
+// How a call's warps and clusters split the sources.
+struct SplitShape {
+  int sw, csize;
+  double cost;  // rounds of resident CTAs x share of the sources each takes
+};
+
+// Every warp does Q queries x n / (sw * csize) sources, and ending a warp's sum
+// takes about as long as 250 sources, 250 more across a cluster.  Of the shapes
+// that leave a lane a group of sources, the one with the least of rounds x
+// (sources of a part + that); below one round of resident CTAs the time does not
+// fall, above it half a round covers the last one's tail.  Measured (us, sw x
+// csize, smooth distance): 1M sources x 997 queries 1x1 6,292, 8x1 720, 8x2 603,
+// 8x8 570 (chosen), 8x16 649; 65,536 x 16,000 1x1 647, 8x1 515 (chosen), 8x2 541;
+// 20,000 x 262,144 1x1 2,470 (chosen 2x1, 2,511), 8x1 2,627.
+inline SplitShape split_shape(long long nq, long long n, int q_per_warp, int ctas_per_sm,
+                              int sm_count) {
+  SplitShape best = {1, 1, -1.0};
+  for (int sw = 1; sw <= kSplitWarps; sw *= 2) {
+    const long long per_cta = (long long)(kSplitWarps / sw) * q_per_warp;
+    for (int c = 1; c <= 16; c *= 2) {
+      const int parts = sw * c;
+      if (parts > 1 && n < (long long)parts * 32 * kSplitGroup) break;
+      // a cluster sits inside one GPC, and a GPC's last SMs may not hold another:
+      // 284, 264 and 224 of 296 CTAs in clusters of 4, 8 and 16
+      const double fit = c <= 2 ? 1.0 : c == 4 ? 0.96 : c == 8 ? 0.89 : 0.757;
+      const double rounds =
+          (double)((nq + per_cta - 1) / per_cta * c) / (sm_count * ctas_per_sm * fit);
+      const double cost =
+          std::max(1.0, rounds + 0.5) * ((double)n / parts + (c > 1 ? 500.0 : 250.0));
+      if (best.cost < 0.0 || cost < best.cost * 0.999) best = {sw, c, cost};
+    }
+  }
+  return best;
+}
+
+template <class Acc, int DIM>
+cudaError_t launch_split(const DevTree& t, const float* q, long long nq, const KParams& kp,
+                         float* out, float* grads, int* contribs, cudaStream_t stream,
+                         const SplitShape& shape) {
+  const long long per_cta = (long long)(kSplitWarps / shape.sw) * Acc::Q;
+  const long long tiles = (nq + per_cta - 1) / per_cta;
+  if (shape.csize > 8) {
+    cudaError_t e = cudaFuncSetAttribute(split_sum_kernel<Acc, DIM>,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * shape.csize), 1, 1);
+  cfg.blockDim = dim3(kSplitThreads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = shape.csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, split_sum_kernel<Acc, DIM>, t, q, nq, kp, shape.sw, out, grads,
+                            contribs);
+}
+
+}  // namespace
+}  // namespace sbh
