@@ -110,7 +110,7 @@ __device__ __forceinline__ float2 norm_from_sq(float2 r2) {
 }
 
 // part += kernel values of source s at the query pair (-nq = negated queries).
-// Same functions as kernel_fast (tasks.cuh), two queries per instruction.
+// kernel_exact's functions with FMA and the MUFU, two queries per instruction.
 // Gravity accumulates +m / (r + 0.1); the caller negates the total.  MODE
 // (smooth distance only): 0 the plain exponential (any alpha), 1 the scaled form
 // 2^(t + 64) on the MUFU, 2 the scaled form on the FP32 pipe (exp2_fma).
