@@ -63,20 +63,19 @@ __global__ void __launch_bounds__(AD_THREADS)
 
 // --------------------------------------------------------------- sampler ---
 
-template <int DIM, int K, class A>
+template <int DIM, int K, class A, bool FEW>
 __global__ void __launch_bounds__(AD_THREADS)
     sbh_grad_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,
-                    const int* __restrict__ order, int samples, unsigned long long seed,
-                    KParams kp, float* __restrict__ out, float* __restrict__ grads,
-                    int* __restrict__ contribs, int* status) {
+                    int samples, unsigned long long seed, KParams kp, float* __restrict__ out, float* __restrict__ grads,
+                    int* __restrict__ contribs, int* status, int group) {
   using V = typename A::V;
   extern __shared__ float s_mem[];
   const int warp = threadIdx.x >> 5;
   const SbhWarpSmem<V> ws = sbh_carve<V>(s_mem + (size_t)warp * sbh_warp_words<V>());
-  const long long units = (nq + 31) / 32;
+  const long long units = (nq + group - 1) / group;
   const long long stride = (long long)gridDim.x * AD_WARPS;
   for (long long u = (long long)blockIdx.x * AD_WARPS + warp; u < units; u += stride)
-    sbh_warp_task<DIM, K, A>(t, qsoa, nq, order, u * 32, min(nq, u * 32 + 32), 0, samples, seed,
+    sbh_warp_task<DIM, K, FEW, A>(t, qsoa, nq, u * group, min(nq, (u + 1) * group), 0, samples, seed,
                              kp, ws, status, out, contribs, nullptr, grads);
 }
 
@@ -418,16 +417,19 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
   }
   using V = typename A::V;
   const size_t smem = (size_t)AD_WARPS * sbh_warp_words<V>() * sizeof(float);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(sbh_grad_kernel<DIM, K, A>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  long long blocks = ((nq + 31) / 32 + AD_WARPS - 1) / AD_WARPS;
+  const int group = sampler_group(nq, sm_count);
+  long long blocks = ((nq + group - 1) / group + AD_WARPS - 1) / AD_WARPS;
   const long long cap = (long long)sm_count * 256;
   if (blocks > cap) blocks = cap;
-  sbh_grad_kernel<DIM, K, A><<<(unsigned)blocks, AD_THREADS, smem, stream>>>(
-      t, q, nq, order, samples, seed, kp, out, grads, contribs, status);
+  const auto kernel = group <= FewQueries<A>::kMax ? sbh_grad_kernel<DIM, K, A, true>
+                                                   : sbh_grad_kernel<DIM, K, A, false>;
+  if (smem > 48 * 1024) {
+    cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  kernel<<<(unsigned)blocks, AD_THREADS, smem, stream>>>(t, q, nq, samples, seed, kp, out, grads,
+                                                         contribs, status, group);
   return cudaGetLastError();
 }
 

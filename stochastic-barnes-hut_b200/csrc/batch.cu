@@ -29,6 +29,7 @@
 #include <cstring>
 
 #include "batch.h"
+#include "launch.h"
 #include "scan.cuh"
 #include "tasks.cuh"
 
@@ -188,14 +189,14 @@ __device__ __forceinline__ void run_bh(const DevTree& t, const BatchItem& it, lo
                                 it.contribs, status, stk, stack_cap, it.self_mass);
 }
 
-template <int DIM, int K>
+template <int DIM, int K, bool FEW>
 __device__ __noinline__ void run_sbh(const DevTree& t, const BatchItem& it, long long u,
-                                        const int* ord, float* scratch, int* status) {
+                                     float* scratch, int* status) {
   const SbhWarpSmem<float> ws = sbh_carve<float>(scratch);
   const long long s0 = u * it.unit_queries;
   const long long s1 = min(it.nq, s0 + it.unit_queries);
   for (long long s = s0; s < s1; s += 32)
-    sbh_warp_task<DIM, K>(t, it.q, it.nq, ord, s, min(s1, s + 32), it.query_base, it.samples,
+    sbh_warp_task<DIM, K, FEW>(t, it.q, it.nq, s, min(s1, s + 32), it.query_base, it.samples,
                           it.seed, it.kp, ws, status, it.out, it.contribs, it.self_mass);
 }
 
@@ -215,7 +216,12 @@ __device__ __forceinline__ void run_unit(const DevTree& t, const BatchItem& it, 
                                          int* status) {
   const int* ord = it.sort_bits > 0 ? order + it.sort_base : nullptr;
   if (CLASS == kClassBh) run_bh<DIM, K>(t, it, u, ord, scratch, stack_cap, status);
-  if (CLASS == kClassSbh) run_sbh<DIM, K>(t, it, u, ord, scratch, status);
+  if (CLASS == kClassSbh) {
+    if (it.unit_queries <= FewQueries<SumF<DIM, K>>::kMax)
+      run_sbh<DIM, K, true>(t, it, u, scratch, status);
+    else
+      run_sbh<DIM, K, false>(t, it, u, scratch, status);
+  }
   if (CLASS == kClassBf) run_bf<DIM, K>(t, it, u, scratch);
 }
 
@@ -434,13 +440,17 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
     if (ca != cb) return ca < cb;
     return unit_cost(a) > unit_cost(b);
   });
+  long long sampled = 0;
+  for (const BatchItem& it : items)
+    if (batch_class(it.method) == kClassSbh) sampled += it.nq;
+  const int sampler_unit = std::min(tuning.sampler_unit, sampler_group(sampled, sm_count_));
   long long sort_base = 0, bucket_base = 0, unit_base[kClasses] = {0, 0, 0};
   for (BatchItem& it : items) {
     if (it.tree < 0 || it.tree >= (int)host_trees.size()) return "request names an unknown tree";
     const DevTree& t = host_trees[it.tree];
     if (t.depth + 2 > lim_.max_tree_depth + 2) return "tree deeper than the engine supports";
     if (t.root_children > lim_.max_root_children) return "tree root wider than the engine supports";
-    const bool sorted = it.method == 1 || it.method == 3;  // vote keeps the caller's order
+    const bool sorted = it.method == 1;  // vote and the sampler keep the caller's order
     it.sort_bits =
         (sorted && it.sort_bits >= 0) ? sort_bits_for(it.nq, t.dim, tuning.bucket_queries) : 0;
     it.dim = t.dim;
@@ -450,10 +460,11 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
     it.bucket_base = bucket_base;
     it.buckets = it.sort_bits > 0 ? (1LL << (t.dim * it.sort_bits)) : 1;
     it.unit_base = unit_base[batch_class(it.method)];
-    // Work unit: sampler queries per warp (tuned); Barnes-Hut queries per warp
+    // Work unit: sampler queries per warp (tuned; fewer in batches of few, as in
+    // a single call); Barnes-Hut queries per warp
     // walk (tuned; vote keeps 32, its acceptance is defined over 32 queries);
     // brute force kBfUnitQueries per warp (query pairs per lane, tasks.cuh).
-    it.unit_queries = it.method == 3   ? tuning.sampler_unit
+    it.unit_queries = it.method == 3   ? sampler_unit
                       : it.method == 1 ? tuning.bh_unit
                       : it.method == 0 ? kBfUnitQueries
                                        : kUnitQueriesWarp;

@@ -74,9 +74,8 @@ inline void bind_tree(sbh_gpu_tree* g, const TreeLayout& L) {
 int clone_gpu_tree(const sbh_gpu_tree* src, sbh_gpu_tree** out);
 
 // Enqueues one stochastic evaluation of a batched request as its own launch of
-// the single-call sampler (query sort with scratch from the library's pool,
-// then stochastic_kernel): device pointers, `self_mass` optional, device
-// bounds reported to `status`, `query_base` the index of d_q's first query in
+// the single-call sampler: device pointers, `self_mass` optional, device bounds
+// reported to `status`, `query_base` the index of d_q's first query in
 // its whole request.  Results equal the batch kernel's for the same request
 // (the random streams are keyed by query index).  The caller has checked the
 // parameters and made the tree's device current.

@@ -24,18 +24,17 @@ using sbh::DeviceGuard;
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Device bytes an evaluation needs besides queries and results: the query
-// order and the sort workspace (0 when the method keeps the given order).
+// The methods whose callers leave the order of evaluation to the library.
 bool wants_sort(const sbh_params* p) {
   if (p->flags & SBH_FLAG_KEEP_ORDER) return false;
   return p->method == SBH_METHOD_BARNES_HUT || p->method == SBH_METHOD_STOCHASTIC;
 }
 
-// Whether a call of nq queries is worth ordering (small Barnes-Hut calls are not).
+// Whether a call of nq queries is worth ordering: Barnes-Hut calls that are not small.
 bool needs_order(const sbh_gpu_tree* tree, const sbh_params* p, int64_t nq) {
-  if (!wants_sort(p)) return false;
-  return !(p->method == SBH_METHOD_BARNES_HUT && !(p->flags & SBH_FLAG_STAGE_LEAVES) &&
-           nq <= sbh::kBhUnorderedQueries && sbh::bh_query_per_warp(nq, tree->sm_count));
+  if (!wants_sort(p) || p->method != SBH_METHOD_BARNES_HUT) return false;
+  return (p->flags & SBH_FLAG_STAGE_LEAVES) || nq > sbh::kBhUnorderedQueries ||
+         !sbh::bh_query_per_warp(nq, tree->sm_count);
 }
 
 // Enqueues one evaluation.  With `grad` the adjoint kernels run instead (values
@@ -71,7 +70,7 @@ cudaError_t run_eval(sbh_gpu_tree* tree, const sbh_params* p, const float* d_q, 
                                     stream, tree->sm_count,
                                     (p->flags & SBH_FLAG_STAGE_LEAVES) != 0);
     case SBH_METHOD_STOCHASTIC:
-      return sbh::launch_stochastic(t, p->kernel, d_q, nq, order, p->samples_per_subdomain,
+      return sbh::launch_stochastic(t, p->kernel, d_q, nq, p->samples_per_subdomain,
                                     p->seed, kp, d_out, d_contribs, tree->d_status, stream,
                                     tree->sm_count);
   }
@@ -346,29 +345,9 @@ int sbh::enqueue_stochastic_direct(const sbh_gpu_tree* tree, const sbh_params& p
   sbh::KParams kp;
   kp.alpha = std::isnan(p.alpha) ? t.alpha : p.alpha;
   kp.eps2 = p.eps * p.eps;
-  void* tmp = nullptr;
-  const int* order = nullptr;
-  if (wants_sort(&p)) {
-    const size_t b_ord = align256((size_t)nq * sizeof(int));
-    cudaMemPool_t pool = nullptr;
-    int st = scratch_pool(tree->device, &pool);
-    if (st != SBH_OK) return st;
-    SBH_CK(cudaMallocFromPoolAsync(&tmp, b_ord + sbh::query_sort_workspace_bytes(nq), pool,
-                                   stream),
-           "cudaMallocFromPoolAsync(workspace)");
-    int* d_ord = static_cast<int*>(tmp);
-    cudaError_t e = sbh::launch_query_sort(d_q, nq, t.dim, static_cast<char*>(tmp) + b_ord,
-                                           d_ord, stream);
-    if (e != cudaSuccess) {
-      cudaFreeAsync(tmp, stream);
-      return cuda_fail(e, "query sort");
-    }
-    order = d_ord;
-  }
-  cudaError_t e = sbh::launch_stochastic(t, p.kernel, d_q, nq, order, p.samples_per_subdomain,
+  cudaError_t e = sbh::launch_stochastic(t, p.kernel, d_q, nq, p.samples_per_subdomain,
                                          p.seed, kp, d_out, d_contribs, d_status, stream,
                                          tree->sm_count, d_self_mass, query_base);
-  if (tmp) cudaFreeAsync(tmp, stream);
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
   return SBH_OK;
 }

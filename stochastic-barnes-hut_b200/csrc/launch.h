@@ -31,14 +31,23 @@ cudaError_t launch_barnes_hut(const DevTree& t, int kernel, bool vote, const flo
                               float* out, int* contribs, int* status, cudaStream_t stream,
                               int sm_count, bool stage_leaves = false);
 
+// Queries a warp of the sampler takes at a time: a power of two up to 32 that
+// leaves 64 to 128 units of work per SM (128 to 256 before 32 are taken; 32 warps
+// of an SM run at once).  A warp's queries run one after the other, so a call lasts
+// at least as long as one unit; sharing the first level among them is worth
+// little by comparison.  Measured on B200 (us, 100,000-point Gaussian mixture, 256
+// paths, groups of 1 / 4 / 8 / 16 / 32): 1,500 queries 131 / 350 / 619 / 1,177 / 2,202;
+// 16,000 453 / 467 / 709 / 1,321 / 2,378; 100,000 2,488 / 2,208 / 2,241 / 2,622 /
+// 3,003; 400,000 10,099 / 8,258 / 8,136 / 8,288 / 8,370.
+int sampler_group(long long nq, int sm_count);
+
 // self_mass (optional, indexed like the queries): subtract each query's own
 // source term, as batched requests may ask.  query_base: index of q[0] within
 // its whole request (keys the random streams of a request split into parts).
 cudaError_t launch_stochastic(const DevTree& t, int kernel, const float* q, long long nq,
-                              const int* order, int samples, unsigned long long seed,
-                              const KParams& kp, float* out, int* contribs, int* status,
-                              cudaStream_t stream, int sm_count,
-                              const float* self_mass = nullptr, long long query_base = 0);
+                              int samples, unsigned long long seed, const KParams& kp,
+                              float* out, int* contribs, int* status, cudaStream_t stream,
+                              int sm_count, const float* self_mass = nullptr, long long query_base = 0);
 
 // Values and query-position gradients (adjoint.cu): method is SBH_METHOD_*,
 // kernel gravity, Plummer or smooth distance; grads is SoA [dim][nq] or null.

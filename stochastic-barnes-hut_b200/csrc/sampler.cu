@@ -12,8 +12,13 @@
 //     continuation probabilities; average the samples.
 //   result = sum of BH terms + sum of averaged corrections.
 //
-// B200 mapping: a warp takes 32 queries at a time (sbh_warp_task, tasks.cuh).
-//   * First level, lane per query.  Every sample of S takes its first step with
+// B200 mapping: a warp takes up to 32 queries at a time (sbh_warp_task, tasks.cuh;
+// fewer in smaller calls, see sampler_group).  The queries keep the caller's
+// order: a query's paths spread over the tree whichever query the next warp
+// holds, and ordering them spatially cost more than its L1 hits gave back
+// at every size (6,000 queries 234 -> 208 us without it, 4M 77.7 -> 77.4 ms).
+//   * First level, lane per query (in warps of up to 16 queries the lanes evaluate
+//     records and a lane per query adds them).  Every sample of S takes its first step with
 //     probability 1 and weight |S| / (1 x |S|) = 1, adding
 //     sum_{children c of S} k(c) - k(S); with S's BH term k(S) that is sum_c k(c)
 //     whatever the sample.  So the first-level part of the estimate is the sum
@@ -63,62 +68,73 @@ constexpr int SBH_WARPS = SBH_THREADS / 32;
 // are keyed by query_base + the query's index, and self_mass (when non-null)
 // subtracts each query's own source term.  Compiled apart so that plain calls
 // carry nothing of it.
-template <int DIM, int K, bool PART>
+template <int DIM, int K, bool PART, bool FEW>
 __global__ void __launch_bounds__(SBH_THREADS, 8)
     stochastic_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,
-                      const int* __restrict__ order, int samples, unsigned long long seed,
+                      int samples, unsigned long long seed,
                       KParams kp, float* __restrict__ out, int* __restrict__ contribs,
-                      int* status, const float* __restrict__ self_mass, long long query_base) {
+                      int* status, const float* __restrict__ self_mass, long long query_base,
+                      int group) {
   extern __shared__ float s_mem[];
   const int warp = threadIdx.x >> 5;
   const SbhWarpSmem<float> ws = sbh_carve<float>(s_mem + (size_t)warp * sbh_warp_words<float>());
-  const long long units = (nq + 31) / 32;
+  const long long units = (nq + group - 1) / group;
   const long long stride = (long long)gridDim.x * SBH_WARPS;
   for (long long u = (long long)blockIdx.x * SBH_WARPS + warp; u < units; u += stride) {
-    sbh_warp_task<DIM, K>(t, qsoa, nq, order, u * 32, min(nq, u * 32 + 32),
+    sbh_warp_task<DIM, K, FEW>(t, qsoa, nq, u * group, min(nq, (u + 1) * group),
                           PART ? query_base : 0, samples, seed, kp, ws, status, out, contribs,
                           PART ? self_mass : nullptr);
   }
 }
 
-template <int DIM, int K, bool PART>
-cudaError_t launch_sbh_variant(const DevTree& t, const float* q, long long nq, const int* order,
+template <int DIM, int K, bool PART, bool FEW>
+cudaError_t launch_sbh_variant(const DevTree& t, const float* q, long long nq,
                        int samples, unsigned long long seed, const KParams& kp, float* out,
                        int* contribs, int* status, cudaStream_t stream, int sm_count,
-                       const float* self_mass, long long query_base) {
+                       const float* self_mass, long long query_base, int group) {
   const size_t smem = (size_t)SBH_WARPS * sbh_warp_words<float>() * sizeof(float);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(stochastic_kernel<DIM, K, PART>,
+    cudaError_t e = cudaFuncSetAttribute(stochastic_kernel<DIM, K, PART, FEW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  // A warp takes 32 queries at a time; blocks beyond the resident ones are
+  // A warp takes `group` queries at a time; blocks beyond the resident ones are
   // handed out as earlier ones finish, which balances uneven query costs.
-  const long long units = (nq + 31) / 32;
+  const long long units = (nq + group - 1) / group;
   long long blocks = (units + SBH_WARPS - 1) / SBH_WARPS;
   const long long cap = (long long)sm_count * 256;
   if (blocks > cap) blocks = cap;
-  stochastic_kernel<DIM, K, PART><<<(unsigned)blocks, SBH_THREADS, smem, stream>>>(
-      t, q, nq, order, samples, seed, kp, out, contribs, status, self_mass, query_base);
+  stochastic_kernel<DIM, K, PART, FEW><<<(unsigned)blocks, SBH_THREADS, smem, stream>>>(
+      t, q, nq, samples, seed, kp, out, contribs, status, self_mass, query_base, group);
   return cudaGetLastError();
 }
 
 template <int DIM, int K>
-cudaError_t launch_sbh(const DevTree& t, const float* q, long long nq, const int* order,
+cudaError_t launch_sbh(const DevTree& t, const float* q, long long nq,
                        int samples, unsigned long long seed, const KParams& kp, float* out,
                        int* contribs, int* status, cudaStream_t stream, int sm_count,
                        const float* self_mass, long long query_base) {
-  if (self_mass || query_base)
-    return launch_sbh_variant<DIM, K, true>(t, q, nq, order, samples, seed, kp, out, contribs,
-                                            status, stream, sm_count, self_mass, query_base);
-  return launch_sbh_variant<DIM, K, false>(t, q, nq, order, samples, seed, kp, out, contribs,
-                                           status, stream, sm_count, self_mass, query_base);
+  const int group = sampler_group(nq, sm_count);
+  const bool few = group <= FewQueries<SumF<DIM, K>>::kMax;
+  const auto launch = self_mass || query_base
+                          ? (few ? launch_sbh_variant<DIM, K, true, true>
+                                 : launch_sbh_variant<DIM, K, true, false>)
+                          : (few ? launch_sbh_variant<DIM, K, false, true>
+                                 : launch_sbh_variant<DIM, K, false, false>);
+  return launch(t, q, nq, samples, seed, kp, out, contribs, status, stream, sm_count, self_mass,
+                query_base, group);
 }
 
 }  // namespace
 
+int sampler_group(long long nq, int sm_count) {
+  int g = 1;
+  while (g < 32 && (long long)g * (g < 16 ? 128 : 256) * sm_count < nq) g *= 2;
+  return g;
+}
+
 cudaError_t launch_stochastic(const DevTree& t, int kernel, const float* q, long long nq,
-                              const int* order, int samples, unsigned long long seed,
+                              int samples, unsigned long long seed,
                               const KParams& kp, float* out, int* contribs, int* status,
                               cudaStream_t stream, int sm_count, const float* self_mass,
                               long long query_base) {
@@ -132,7 +148,7 @@ cudaError_t launch_stochastic(const DevTree& t, int kernel, const float* q, long
   }
 #define SBH_SBH_CASE(D, K)      \
   if (t.dim == D && kernel == K) \
-    return launch_sbh<D, K>(t, q, nq, order, samples, seed, kp, out, contribs, status, stream, \
+    return launch_sbh<D, K>(t, q, nq, samples, seed, kp, out, contribs, status, stream, \
                             sm_count, self_mass, query_base);
   SBH_SBH_CASE(3, kGravity)
   SBH_SBH_CASE(3, kWindingNumber)

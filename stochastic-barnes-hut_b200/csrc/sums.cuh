@@ -9,7 +9,10 @@
 //   SumGrad<DIM, K>  gravity or Plummer value plus its query-position gradient.
 //                    The value is rounded exactly as SumF rounds it, so it equals
 //                    the plain evaluation bit for bit; the gradient is an
-//                    ordinary FP32 sum of the terms' analytic gradients.
+//                    ordinary FP32 sum of the terms' analytic gradients, each
+//                    rounded before it is added and without contractions left
+//                    to the compiler, so that sums of the same terms in the same
+//                    order agree bit for bit whichever routine forms them.
 //   SumLse<DIM>      smooth distance in max-shifted form.  (m, s, g) stands for
 //                    the sum e^m * s of exp(-alpha r) terms and for its gradient
 //                    e^m * g; adding two values rescales the one with the smaller
@@ -78,7 +81,7 @@ struct SumGrad {
   static constexpr bool kOrdered = true;
   __device__ __forceinline__ static float ordered(V a) { return a.v; }
   __device__ __forceinline__ static V add_rest(V a, V b) {
-    return V{a.v, a.gx + b.gx, a.gy + b.gy, a.gz + b.gz};
+    return V{a.v, radd(a.gx, b.gx), radd(a.gy, b.gy), radd(a.gz, b.gz)};
   }
   __device__ __forceinline__ static V join(float sum, V rest) {
     return V{sum, rest.gx, rest.gy, rest.gz};
@@ -89,13 +92,13 @@ struct SumGrad {
     return V{n, n, n, n};
   }
   __device__ __forceinline__ static V add(V a, V b) {
-    return V{radd(a.v, b.v), a.gx + b.gx, a.gy + b.gy, a.gz + b.gz};
+    return V{radd(a.v, b.v), radd(a.gx, b.gx), radd(a.gy, b.gy), radd(a.gz, b.gz)};
   }
   __device__ __forceinline__ static V sub(V a, V b) {
-    return V{rsub(a.v, b.v), a.gx - b.gx, a.gy - b.gy, a.gz - b.gz};
+    return V{rsub(a.v, b.v), rsub(a.gx, b.gx), rsub(a.gy, b.gy), rsub(a.gz, b.gz)};
   }
   __device__ __forceinline__ static V scale(float w, V a) {
-    return V{rmul(w, a.v), w * a.gx, w * a.gy, w * a.gz};
+    return V{rmul(w, a.v), rmul(w, a.gx), rmul(w, a.gy), rmul(w, a.gz)};
   }
   __device__ __forceinline__ static V div(V a, float d) {
     return V{rdiv(a.v, d), a.gx / d, a.gy / d, a.gz / d};
@@ -113,7 +116,7 @@ struct SumGrad {
   __device__ __forceinline__ static V point(float4 pm, float4 nr, float3 q, const KParams& kp) {
     const float v = kernel_exact<DIM, K>(pm, nr, q, kp);
     const float dx = pm.x - q.x, dy = pm.y - q.y, dz = DIM == 3 ? pm.z - q.z : 0.f;
-    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float r2 = fmaf(dz, dz, fmaf(dy, dy, rmul(dx, dx)));
     float c;
     if (K == kGravity) {
       const float r = sqrtf(r2), rs = r + 1e-1f;
@@ -122,7 +125,7 @@ struct SumGrad {
       const float s = r2 + kp.eps2;
       c = pm.w / (s * sqrtf(s));
     }
-    return V{v, c * dx, c * dy, c * dz};
+    return V{v, rmul(c, dx), rmul(c, dy), rmul(c, dz)};
   }
   __device__ __forceinline__ static V node(float4 cm, float4 agg, float3 q, const KParams& kp) {
     return point(make_float4(cm.x, cm.y, cm.z, agg.x), make_float4(agg.y, agg.z, agg.w, 0.f), q,
@@ -168,13 +171,14 @@ struct SumLse {
     }
     if (b.m == -__int_as_float(0x7f800000)) return a;  // b is zero (and so is a if equal)
     const float f = expf(b.m - a.m);
-    return V{a.m, a.s + f * b.s, a.gx + f * b.gx, a.gy + f * b.gy, a.gz + f * b.gz};
+    return V{a.m, fmaf(f, b.s, a.s), fmaf(f, b.gx, a.gx), fmaf(f, b.gy, a.gy),
+             fmaf(f, b.gz, a.gz)};
   }
   __device__ __forceinline__ static V sub(V a, V b) {
     return add(a, V{b.m, -b.s, -b.gx, -b.gy, -b.gz});
   }
   __device__ __forceinline__ static V scale(float w, V a) {
-    return V{a.m, w * a.s, w * a.gx, w * a.gy, w * a.gz};
+    return V{a.m, rmul(w, a.s), rmul(w, a.gx), rmul(w, a.gy), rmul(w, a.gz)};
   }
   __device__ __forceinline__ static V div(V a, float d) {
     return V{a.m, a.s / d, a.gx / d, a.gy / d, a.gz / d};
@@ -194,7 +198,7 @@ struct SumLse {
     // The exponent exactly as the plain kernel forms it (include/kernel.h:55-58).
     const float r = rsqrt_ieee(dot_exact<DIM>(dx, dy, dz, dx, dy, dz));
     const float c = r > 0.f ? kp.alpha / r : 0.f;
-    return V{rmul(-kp.alpha, r), 1.f, c * dx, c * dy, c * dz};
+    return V{rmul(-kp.alpha, r), 1.f, rmul(c, dx), rmul(c, dy), rmul(c, dz)};
   }
   __device__ __forceinline__ static V node(float4 cm, float4 agg, float3 q, const KParams& kp) {
     return point(make_float4(cm.x, cm.y, cm.z, agg.x), make_float4(agg.y, agg.z, agg.w, 0.f), q,

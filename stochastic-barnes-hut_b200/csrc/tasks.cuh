@@ -542,6 +542,9 @@ struct SbhWarpSmem {
   // [32][8] records staged for the first-level sum: (x, y, z, mass), (normal,
   // flag); flag < 0 marks a leaf whose points are summed instead
   __device__ __forceinline__ float4* tile() const { return reinterpret_cast<float4*>(base + 288); }
+  // a row of terms per query where the warp holds few (FewQueries; over the tile
+  // and the queue below, both unused meanwhile)
+  __device__ __forceinline__ V* terms() const { return reinterpret_cast<V*>(base + 288); }
   // [kQueue][kEntry] surviving paths: path index, sampled point, node to
   // expand, next node, path probability, running ratio, next node's depth,
   // pending random word
@@ -627,6 +630,82 @@ __device__ __forceinline__ long long sum_records(const DevTree& t, long long b, 
     }
   }
   __syncwarp();
+  return cnt;
+}
+
+// The same sum for a warp that holds few queries (lane k < g its query k's): every
+// lane evaluates one record for each query in turn, the terms wait in shared
+// memory (`terms`, a row per query) and lane k adds its row in record order, so
+// the sum is sum_records' bit for bit.
+template <class A>
+struct FewQueries {
+  using V = typename A::V;
+  static constexpr bool kOneWord = sizeof(V) == 4;
+  static constexpr int kMax = kOneWord ? 16 : 4;      // queries
+  static constexpr int kStride = kOneWord ? 36 : 33;  // values per row (rows 4 banks apart)
+  static constexpr int kWords = kMax * kStride * (int)(sizeof(V) / 4);
+};
+
+template <bool NODES, class A>
+__device__ __forceinline__ long long sum_records_few(const DevTree& t, long long b, long long e,
+                                                     int g, float3 q, const KParams& kp,
+                                                     typename A::V* terms, typename A::V& acc) {
+  using V = typename A::V;
+  constexpr int kStride = FewQueries<A>::kStride;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  long long cnt = 0;
+  float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+  auto fetch = [&](long long base) {
+    const long long i = base + lane;
+    if (i < e) {
+      r0 = NODES ? __ldg(t.nd_cm + i) : __ldg(t.pt_pm + i);
+      r1 = NODES ? __ldg(t.nd_agg + i) : __ldg(t.pt_nrm + i);
+    }
+  };
+  fetch(b);
+  for (long long base = b; base < e; base += 32) {
+    const int n = (int)min(32LL, e - base);
+    const float4 c0 = r0, c1 = r1;
+    fetch(base + 32);
+    if (NODES && __any_sync(full, lane < n && c0.w < 0.f)) {
+      // some record is a leaf holding several points (or none)
+      for (int r = 0; r < n; r++) {
+        const float4 cm = __ldg(t.nd_cm + base + r), ag = __ldg(t.nd_agg + base + r);
+        if (cm.w < 0.f) {
+          const int4 tc = __ldg(t.nd_topo + base + r);
+          if (lane < g)
+            for (int i = tc.z; i < tc.w; i++)
+              acc = A::add(acc, A::point(__ldg(t.pt_pm + i), __ldg(t.pt_nrm + i), q, kp));
+          cnt += tc.w - tc.z;
+        } else {
+          if (lane < g) acc = A::add(acc, A::node(cm, ag, q, kp));
+          cnt++;
+        }
+      }
+      continue;
+    }
+    for (int k = 0; k < g; k++) {
+      const float3 qk = make_float3(__shfl_sync(full, q.x, k), __shfl_sync(full, q.y, k),
+                                    __shfl_sync(full, q.z, k));
+      if (lane < n) terms[k * kStride + lane] = NODES ? A::node(c0, c1, qk, kp)
+                                                      : A::point(c0, c1, qk, kp);
+    }
+    __syncwarp();
+    if (lane < g) {
+      const V* row = terms + lane * kStride;
+      int r = 0;
+      if constexpr (FewQueries<A>::kOneWord) {
+        for (; r + 4 <= n; r += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(row + r);
+          acc = A::add(A::add(A::add(A::add(acc, x.x), x.y), x.z), x.w);
+        }
+      }
+      for (; r < n; r++) acc = A::add(acc, row[r]);
+    }
+    cnt += n;
+    __syncwarp();
+  }
   return cnt;
 }
 
@@ -727,14 +806,16 @@ __device__ __forceinline__ int sbh_round(const DevTree& t, float3 q, long long k
 }
 
 // The stochastic estimator (multiLevelPrefixControlVariateSample_stackless,
-// include/tree_sampler.h:21-113) for the queries at sorted positions
-// [slot0, slot_end) (at most 32), one warp: see sampler.cu for the method.
+// include/tree_sampler.h:21-113) for the queries [slot0, slot_end) (at
+// most 32), one warp: see sampler.cu for the method.
 // The random streams of query qi are keyed by key_base + qi (its index within
 // its request).  Results go to out/grads (policy A) and contribs, with each
-// query's own source term subtracted when self_mass is given.
-template <int DIM, int K, class A = SumF<DIM, K>>
+// query's own source term subtracted when self_mass is given.  FEW: at most
+// FewQueries<A>::kMax queries, the first level summed by sum_records_few (same
+// results; compiled apart, since both forms in one kernel cost it registers).
+template <int DIM, int K, bool FEW, class A = SumF<DIM, K>>
 __device__ __forceinline__ void sbh_warp_task(
-    const DevTree& t, const float* __restrict__ qsoa, long long nq, const int* __restrict__ order,
+    const DevTree& t, const float* __restrict__ qsoa, long long nq,
     long long slot0, long long slot_end, long long key_base, int samples,
     unsigned long long seed, const KParams& kp, const SbhWarpSmem<typename A::V>& ws,
     int* status, float* __restrict__ out, int* __restrict__ contribs,
@@ -746,11 +827,6 @@ __device__ __forceinline__ void sbh_warp_task(
   if (nqw <= 0) return;
   const int R = t.root_children;
   const int c0 = __ldg(t.nd_topo).x;
-  // The lane's own query (lane < nqw), reloaded where needed rather than
-  // carried through the path loop.
-  auto query_index = [&](int l) -> long long {
-    return order ? (long long)__ldg(order + slot0 + l) : slot0 + l;
-  };
 
   // ---- First level, lane per query.  Every path's first step leaves its
   // subdomain S with probability 1 and weight |S| / (1 x |S|) = 1 and adds
@@ -763,7 +839,7 @@ __device__ __forceinline__ void sbh_warp_task(
   V acc = A::zero();
   long long cntA = 0;
   {
-  const float3 q = lane < nqw ? load_query<DIM>(qsoa, nq, query_index(lane))
+  const float3 q = lane < nqw ? load_query<DIM>(qsoa, nq, slot0 + lane)
                               : make_float3(0.f, 0.f, 0.f);
   int l2b = 0x7fffffff, l2e = -1, nint = 0;
   long long l2n = 0;
@@ -779,7 +855,8 @@ __device__ __forceinline__ void sbh_warp_task(
     for (unsigned m = __ballot_sync(full, j < R && !internal); m != 0u; m &= m - 1u) {
       const int b = __ffs(m) - 1;
       const int z = __shfl_sync(full, tS.z, b), w = __shfl_sync(full, tS.w, b);
-      cntA += sum_records<false, A>(t, z, w, q, kp, ws.tile(), acc);
+      cntA += FEW ? sum_records_few<false, A>(t, z, w, nqw, q, kp, ws.terms(), acc)
+                  : sum_records<false, A>(t, z, w, q, kp, ws.tile(), acc);
     }
   }
 #pragma unroll
@@ -791,8 +868,10 @@ __device__ __forceinline__ void sbh_warp_task(
   bool layout_ok = true;
   if (nint > 0) {
     layout_ok = l2n == (long long)l2e - l2b;
-    if (layout_ok) cntA += (long long)samples * sum_records<true, A>(t, l2b, l2e, q, kp,
-                                                                        ws.tile(), acc);
+    if (layout_ok)
+      cntA += (long long)samples *
+              (FEW ? sum_records_few<true, A>(t, l2b, l2e, nqw, q, kp, ws.terms(), acc)
+                   : sum_records<true, A>(t, l2b, l2e, q, kp, ws.tile(), acc));
     cntA += nint;  // each internal subdomain's Barnes-Hut term
   }
   if (!layout_ok && lane == 0) report_status(status, kStatusNullChild);
@@ -805,7 +884,7 @@ __device__ __forceinline__ void sbh_warp_task(
   // ---- Deeper steps, one query at a time, lanes over its R x samples paths.
   const int P = R * samples;
   for (int k = 0; k < nqw; k++) {
-    const long long qik = query_index(k);
+    const long long qik = slot0 + k;
     const float3 qk = load_query<DIM>(qsoa, nq, qik);
     const long long key = key_base + qik;
     bool poisoned = false;
@@ -911,7 +990,7 @@ __device__ __forceinline__ void sbh_warp_task(
   }
 
   if (lane < nqw) {
-    const long long qi = query_index(lane);
+    const long long qi = slot0 + lane;
     V r = R == 0 ? A::zero() : A::add(ws.qacc()[lane], A::div(ws.qsum()[lane], (float)samples));
     if (ws.qflag()[lane] & 1) r = A::nan();
     if (self_mass) {
