@@ -18,9 +18,7 @@ struct sbh_gpu_tree {
   size_t bytes = 0;
   int* d_status = nullptr;
   sbh_tree_info info = {};
-  std::mutex mu;        // serialises blocking calls (they share `ws`)
-  void* ws = nullptr;   // workspace of blocking calls
-  size_t ws_bytes = 0;
+  std::mutex mu;        // serialises blocking calls (they share the events)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -69,6 +67,13 @@ inline void bind_tree(sbh_gpu_tree* g, const TreeLayout& L) {
   t.nd_mask = reinterpret_cast<const unsigned long long*>(base + L.mask);
   t.pt_code = reinterpret_cast<const unsigned long long*>(base + L.code);
 }
+
+// The library's memory pool on `device` (stream-ordered scratch).
+int scratch_pool(int device, cudaMemPool_t* out);
+
+// Whether `device` (a valid index) runs this build's code; its SM count.  Two
+// attribute reads: the whole property record takes the driver 2.5 ms.
+int check_device(int device, int* sm_count);
 
 // A copy of a device tree (its own allocation and status word), on its device.
 int clone_gpu_tree(const sbh_gpu_tree* src, sbh_gpu_tree** out);

@@ -77,37 +77,6 @@ cudaError_t run_eval(sbh_gpu_tree* tree, const sbh_params* p, const float* d_q, 
   return cudaErrorInvalidValue;
 }
 
-// Stream-ordered scratch of the asynchronous entry points comes from a pool of
-// the library's own per device, which keeps freed memory reserved (release
-// threshold: unlimited): a process's default pool hands memory back to the
-// driver at every synchronisation, so each call would map its scratch afresh.
-std::mutex g_pool_mu;
-cudaMemPool_t g_pools[64] = {};
-
-int scratch_pool(int device, cudaMemPool_t* out) {
-  if (device < 0 || device >= 64) return sbh::fail(SBH_ERR_UNSUPPORTED, "device index beyond 64");
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (!g_pools[device]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    if (e != cudaSuccess) return sbh::cuda_fail(e, "cudaMemPoolCreate(scratch)");
-    uint64_t keep = UINT64_MAX;
-    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return sbh::cuda_fail(e, "cudaMemPoolSetAttribute(scratch)");
-    }
-    g_pools[device] = pool;
-  }
-  *out = g_pools[device];
-  return SBH_OK;
-}
-
 // Extra checks of the gradient entry points.
 int check_grad_params(const sbh_gpu_tree* tree, const sbh_params* p) {
   if (p->kernel == SBH_KERNEL_WINDING_NUMBER)
@@ -137,17 +106,26 @@ int blocking_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* que
   const size_t b_out = align256((size_t)nq * sizeof(float));
   const size_t b_grad = grads ? b_q : 0;
   const size_t b_cnt = contribs ? align256((size_t)nq * sizeof(int)) : 0;
-  const size_t b_ord = align256((size_t)nq * sizeof(int));
-  const size_t b_sort = align256(sbh::query_sort_workspace_bytes(nq));
+  const bool order = needs_order(tree, params, nq);
+  const size_t b_ord = order ? align256((size_t)nq * sizeof(int)) : 0;
+  const size_t b_sort = order ? align256(sbh::query_sort_workspace_bytes(nq)) : 0;
   const size_t need = b_q + b_out + b_grad + b_cnt + b_ord + b_sort;
-  if (tree->ws_bytes < need) {
-    if (tree->ws) cudaFree(tree->ws);
-    tree->ws = nullptr;
-    tree->ws_bytes = 0;
-    SBH_CK(cudaMalloc(&tree->ws, need), "cudaMalloc(workspace)");
-    tree->ws_bytes = need;
-  }
-  char* w = static_cast<char*>(tree->ws);
+  // From the pool (a cudaMalloc on a tree's first call and a cudaFree with the
+  // tree would take 0.35 ms each).
+  cudaMemPool_t pool = nullptr;
+  st = sbh::scratch_pool(tree->device, &pool);
+  if (st != SBH_OK) return st;
+  struct Scratch {
+    void* mem = nullptr;
+    cudaStream_t stream;
+    ~Scratch() {
+      if (mem) cudaFreeAsync(mem, stream);
+    }
+  } scratch;
+  scratch.stream = stream;
+  SBH_CK(cudaMallocFromPoolAsync(&scratch.mem, need, pool, stream),
+         "cudaMallocFromPoolAsync(workspace)");
+  char* w = static_cast<char*>(scratch.mem);
   float* d_q = reinterpret_cast<float*>(w);
   float* d_out = reinterpret_cast<float*>(w + b_q);
   float* d_grad = grads ? reinterpret_cast<float*>(w + b_q + b_out) : nullptr;
@@ -202,7 +180,7 @@ int device_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* d_que
   if (needs_order(tree, params, nq)) {
     const size_t b_ord = align256((size_t)nq * sizeof(int));
     cudaMemPool_t pool = nullptr;
-    st = scratch_pool(tree->device, &pool);
+    st = sbh::scratch_pool(tree->device, &pool);
     if (st != SBH_OK) return st;
     SBH_CK(cudaMallocFromPoolAsync(&tmp, b_ord + sbh::query_sort_workspace_bytes(nq), pool,
                                    stream),
@@ -219,6 +197,51 @@ int device_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* d_que
 
 }  // namespace
 
+// Stream-ordered scratch of the asynchronous entry points comes from a pool of
+// the library's own per device, which keeps freed memory reserved (release
+// threshold: unlimited): a process's default pool hands memory back to the
+// driver at every synchronisation, so each call would map its scratch afresh.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pools[64] = {};
+
+int sbh::scratch_pool(int device, cudaMemPool_t* out) {
+  if (device < 0 || device >= 64) return sbh::fail(SBH_ERR_UNSUPPORTED, "device index beyond 64");
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pools[device]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return sbh::cuda_fail(e, "cudaMemPoolCreate(scratch)");
+    uint64_t keep = UINT64_MAX;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return sbh::cuda_fail(e, "cudaMemPoolSetAttribute(scratch)");
+    }
+    g_pools[device] = pool;
+  }
+  *out = g_pools[device];
+  return SBH_OK;
+}
+
+int sbh::check_device(int device, int* sm_count) {
+  int major = 0, minor = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(sm_count, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return sbh::cuda_fail(e, "cudaDeviceGetAttribute");
+  if (major != 10 || minor != 0)
+    return sbh::fail(SBH_ERR_NO_DEVICE, "this build carries sm_100a code only; device is sm_" +
+                                            std::to_string(major) + std::to_string(minor));
+  return SBH_OK;
+}
+
 SBH_API int sbh_gpu_tree_create(const sbh_host_tree* host, int device, sbh_gpu_tree** out) {
   if (!out) return sbh::fail(SBH_ERR_INVALID_ARGUMENT, "out must be non-null");
   *out = nullptr;
@@ -232,12 +255,9 @@ SBH_API int sbh_gpu_tree_create(const sbh_host_tree* host, int device, sbh_gpu_t
     return sbh::fail(SBH_ERR_NO_DEVICE, "no CUDA device is visible");
   }
   if (device < 0 || device >= ndev) return sbh::fail(SBH_ERR_NO_DEVICE, "device index out of range");
-  cudaDeviceProp prop;
-  SBH_CK(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties");
-  if (prop.major != 10 || prop.minor != 0)
-    return sbh::fail(SBH_ERR_NO_DEVICE,
-                     std::string("this build carries sm_100a code only; device is ") + prop.name +
-                         " (sm_" + std::to_string(prop.major) + std::to_string(prop.minor) + ")");
+  int sm_count = 0;
+  const int st = sbh::check_device(device, &sm_count);
+  if (st != SBH_OK) return st;
   DeviceGuard guard(device);
 
   const int64_t n = h.n, nn = h.nn;
@@ -280,7 +300,7 @@ SBH_API int sbh_gpu_tree_create(const sbh_host_tree* host, int device, sbh_gpu_t
   sbh_gpu_tree* g = new (std::nothrow) sbh_gpu_tree();
   if (!g) return sbh::fail(SBH_ERR_OUT_OF_MEMORY, "host allocation failed");
   g->device = device;
-  g->sm_count = prop.multiProcessorCount;
+  g->sm_count = sm_count;
   g->bytes = L.bytes;
   cudaError_t e = cudaMalloc(&g->mem, L.bytes);
   if (e != cudaSuccess) {
@@ -387,7 +407,6 @@ SBH_API void sbh_gpu_tree_destroy(sbh_gpu_tree* tree) {
   {
     DeviceGuard guard(tree->device);
     cudaDeviceSynchronize();
-    if (tree->ws) cudaFree(tree->ws);
     if (tree->mem) cudaFree(tree->mem);
     if (tree->ev0) cudaEventDestroy(tree->ev0);
     if (tree->ev1) cudaEventDestroy(tree->ev1);
