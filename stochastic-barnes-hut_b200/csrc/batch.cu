@@ -11,14 +11,15 @@
 //                         request's buckets follow the previous request's, so
 //                         the scan also places every request at its offset);
 //   batch_scatter_kernel  the sorted position of every query;
-//   batch_eval_kernel<C>  three persistent kernels, one per method class
-//                         (Barnes-Hut, sampler, brute force), as parallel
+//   batch_eval_kernel<C>, batch_bf_kernel<D, K>
+//                         a persistent kernel per class the batch has (Barnes-Hut,
+//                         sampler, each kind of brute force), as parallel
 //                         branches of the graph: warps take that class's work
 //                         units from its atomic counter and run the same device
-//                         routines as the single-call kernels (tasks.cuh),
-//                         dispatching on kernel and dimension per unit.  Each
-//                         is compiled for its own method alone, so none carries
-//                         the registers or the call overhead of the others.
+//                         routines as the single-call kernels (tasks.cuh,
+//                         lane_sum.cuh), the traversals dispatching on kernel and
+//                         dimension per unit.  Each is compiled for its own work
+//                         alone, so none carries the registers of the others.
 //
 // Every launch parameter of the graph is fixed (grids are persistent; sizes and
 // the request table live in device memory, refreshed by one host-to-device copy
@@ -201,13 +202,85 @@ __device__ __noinline__ void run_sbh(const DevTree& t, const BatchItem& it, long
 }
 
 template <int DIM, int K>
+__device__ __noinline__ void run_bh_query(const DevTree& t, const BatchItem& it, long long u,
+                                          const int* ord, char* scratch, int* status) {
+  const long long s1 = min(it.nq, (u + 1) * it.unit_queries);
+  for (long long s = u * it.unit_queries; s < s1; s++)
+    bh_query_task<DIM, K>(t, it.q, it.nq, ord ? (long long)__ldg(ord + s) : s, it.beta, it.kp,
+                          it.out, it.contribs, status, scratch, it.self_mass);
+}
+
+// Brute force: a tile of kBfTileQueries queries against all parts of the sources
+// (bf_parts), or, of a split request, against one of them; one warp
+// (lane_sum.cuh).  The sums of one part go to `partials` ([tile][part][query]) and
+// the tile's last unit, by its counter, merges them in part order and stores; it
+// leaves the counter at zero.  `tot` is the warp's scratch of kBfTileQueries
+// sums.  The request's fields are read where they are needed, not carried
+// through the sums' registers.
+template <int DIM, int K>
 __device__ __forceinline__ void run_bf(const DevTree& t, const BatchItem& it, long long u,
-                                       float* scratch) {
-  const long long s0 = u * kBfUnitQueries;
-  SrcPair* src = reinterpret_cast<SrcPair*>(scratch);
-  NrmPair* nrm = reinterpret_cast<NrmPair*>(src + 32);
-  bf_warp_task<DIM, K>(t, it.q, it.nq, s0, min(it.nq, s0 + kBfUnitQueries), it.kp, it.out,
-                       it.contribs, it.self_mass, src, nrm);
+                                       PlainSum* tot, PlainSum* partials, unsigned* counters) {
+  using Acc = PlainAcc<DIM, K, kBfTileQueries / 2>;
+  const int lane = threadIdx.x & 31;
+  const int split = it.split;
+  const int tile = split ? (int)(u / split) : (int)u;
+  const int part = split ? (int)(u - (long long)tile * split) : -1;
+  const int p1 = split ? part + 1 : bf_parts(t.n);
+  for (int p = split ? part : 0; p < p1; p++) {
+    Acc acc;
+    acc.load(it.q, it.nq, (long long)tile * kBfTileQueries, it.kp);
+    const long long len = bf_part_sources(t.n);
+    sum_range<Acc, !Acc::kNormals>(acc, t.pt_pm, t.pt_nrm, min(p * len, t.n),
+                                   min((p + 1) * len, t.n));
+#pragma unroll
+    for (int j = 0; j < kBfTileQueries; j++) {
+      PlainSum v = merge_lanes(acc.sum(j));
+      if (lane == 0) {
+        if (it.split == 0 && p > 0) {
+          const PlainSum part_sum = v;
+          v = tot[j];
+          v.merge(part_sum);
+        }
+        tot[j] = v;
+      }
+    }
+  }
+  __syncwarp();
+  PlainSum v = tot[lane & (kBfTileQueries - 1)];
+  if (it.split) {
+    // [part][query] sums of the tile; a lane per query
+    float2* sums = reinterpret_cast<float2*>(partials + it.partial_base +
+                                             (long long)tile * it.split * kBfTileQueries);
+    unsigned* counter = counters + it.counter_base + tile;
+    if (lane < kBfTileQueries) {
+      __stcg(sums + part * kBfTileQueries + lane, make_float2(v.hi, v.lo));
+      __threadfence();  // this part's sums before the count that announces them
+    }
+    __syncwarp();
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(counter, 1u);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before + 1 != (unsigned)it.split) return;
+    __threadfence();
+    if (lane == 0) *counter = 0u;
+    for (int p = 0; p < it.split; p++) {
+      const float2 x = __ldcg(sums + p * kBfTileQueries + (lane & (kBfTileQueries - 1)));
+      const PlainSum y = {x.x, x.y};
+      if (p == 0)
+        v = y;
+      else
+        v.merge(y);
+    }
+  }
+  const long long qi = (long long)tile * kBfTileQueries + lane;
+  if (lane < kBfTileQueries && qi < it.nq) {
+    float r = v.hi + v.lo;
+    if (K == kGravity) r = -r;  // accumulate2 adds +m / (r + 0.1)
+    if (it.self_mass)
+      r -= self_term<DIM, K>(load_query<DIM>(it.q, it.nq, qi), __ldg(it.self_mass + qi), it.kp);
+    it.out[qi] = r;
+    if (it.contribs) it.contribs[qi] = (int)t.n;
+  }
 }
 
 template <int CLASS, int DIM, int K>
@@ -215,14 +288,18 @@ __device__ __forceinline__ void run_unit(const DevTree& t, const BatchItem& it, 
                                          const int* order, float* scratch, int stack_cap,
                                          int* status) {
   const int* ord = it.sort_bits > 0 ? order + it.sort_base : nullptr;
-  if (CLASS == kClassBh) run_bh<DIM, K>(t, it, u, ord, scratch, stack_cap, status);
+  if (CLASS == kClassBh) {
+    if (it.per_query)
+      run_bh_query<DIM, K>(t, it, u, ord, reinterpret_cast<char*>(scratch), status);
+    else
+      run_bh<DIM, K>(t, it, u, ord, scratch, stack_cap, status);
+  }
   if (CLASS == kClassSbh) {
     if (it.unit_queries <= FewQueries<SumF<DIM, K>>::kMax)
       run_sbh<DIM, K, true>(t, it, u, scratch, status);
     else
       run_sbh<DIM, K, false>(t, it, u, scratch, status);
   }
-  if (CLASS == kClassBf) run_bf<DIM, K>(t, it, u, scratch);
 }
 
 template <int CLASS>
@@ -242,34 +319,23 @@ __device__ __forceinline__ void dispatch_unit(const DevTree& t, const BatchItem&
   }
 }
 
-// The persistent kernel of one method class: warps take that class's work
-// units from its counter and run them.  Minimum CTAs per SM: the single-call
-// kernels' occupancy (sampler 8 at 64 registers, Barnes-Hut 10 at 48); brute
-// force 4 (at most 128 registers; its unbounded 132 gave 3 CTAs per SM and
-// measured 6% slower).
-template <int CLASS>
-__global__ void __launch_bounds__(kEvalThreads, CLASS == kClassSbh  ? 8
-                                                : CLASS == kClassBh ? 10
-                                                                    : 4)
-    batch_eval_kernel(BatchHeader* hdr, const BatchItem* __restrict__ items,
-                      const DevTree* __restrict__ trees, const int* __restrict__ order,
-                      int* status, int warp_words, int stack_cap) {
-  extern __shared__ float4 s_eval[];
+// A warp's turn through a class's work units: takes them from the class's counter
+// and calls run(tree, item, unit) with the unit's tree and request records, which
+// it keeps in the warp's shared memory (`wbase`), where the walks read them
+// instead of holding them in registers.
+template <class Run>
+__device__ __forceinline__ void for_each_unit(BatchHeader* hdr, const BatchItem* __restrict__ items,
+                                              const DevTree* __restrict__ trees, int cls,
+                                              float* wbase, const Run& run) {
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  float* wbase = reinterpret_cast<float*>(s_eval) + (size_t)warp * warp_words;
-  // Per-warp shared memory: the current tree record, the current request,
-  // then the class's scratch.  The walks read both records from there instead
-  // of holding them in registers.
   const DevTree& ts = *reinterpret_cast<const DevTree*>(wbase);
   const BatchItem& it = *reinterpret_cast<const BatchItem*>(wbase + kTreeWords);
-  float* scratch = wbase + kTreeWords + kItemWords;
-  const int ib = hdr->item_begin[CLASS], ie = hdr->item_end[CLASS];
-  const long long total = hdr->total_units[CLASS];
+  const int ib = hdr->item_begin[cls], ie = hdr->item_end[cls];
+  const long long total = hdr->total_units[cls];
   int cached_tree = -1, cached_item = -1;
   for (;;) {
     unsigned long long unit = 0;
-    if (lane == 0) unit = atomicAdd(&hdr->next_unit[CLASS], 1ull);
+    if (lane == 0) unit = atomicAdd(&hdr->next_unit[cls], 1ull);
     unit = __shfl_sync(0xffffffffu, unit, 0);
     if ((long long)unit >= total) break;
     const int item = ib + find_item_by(items + ib, ie - ib, (long long)unit, &BatchItem::unit_base);
@@ -290,54 +356,88 @@ __global__ void __launch_bounds__(kEvalThreads, CLASS == kClassSbh  ? 8
       cached_tree = tree;
       __syncwarp();
     }
-    const long long u = (long long)unit - it.unit_base;
-    if constexpr (CLASS != kClassBf) {
-      // The traversals read the record from shared memory: a register copy
-      // costs them occupancy (Barnes-Hut) or spills (sampler).
-      dispatch_unit<CLASS>(ts, it, u, order, scratch, stack_cap, status);
-    } else {
-      // Brute force keeps it in registers.
-      const DevTree t = ts;
-      dispatch_unit<CLASS>(t, it, u, order, scratch, stack_cap, status);
-    }
+    run(ts, it, (long long)unit - it.unit_base);
     __syncwarp();
   }
 }
 
+// The persistent kernel of a traversal class.  Minimum CTAs per SM: the
+// single-call kernels' occupancy (sampler 8 at 64 registers, Barnes-Hut 10 at 48).
+template <int CLASS>
+__global__ void __launch_bounds__(kEvalThreads, CLASS == kClassSbh ? 8 : 10)
+    batch_eval_kernel(BatchHeader* hdr, const BatchItem* __restrict__ items,
+                      const DevTree* __restrict__ trees, const int* __restrict__ order,
+                      int* status, int warp_words, int stack_cap) {
+  extern __shared__ float4 s_eval[];
+  float* wbase = reinterpret_cast<float*>(s_eval) + (size_t)(threadIdx.x >> 5) * warp_words;
+  float* scratch = wbase + kTreeWords + kItemWords;
+  for_each_unit(hdr, items, trees, CLASS, wbase,
+                [&](const DevTree& t, const BatchItem& it, long long u) {
+                  dispatch_unit<CLASS>(t, it, u, order, scratch, stack_cap, status);
+                });
+}
+
+// The persistent kernel of one kind of brute force, 16 warps per SM as the single
+// call's: in one kernel for all eight kinds the sums spilled 1 KB a thread, and
+// 200,000 queries x 1M sources took 125 ms (smooth distance) instead of 95.  With
+// 64 queries a warp against all sources in turn (sources staged in shared memory)
+// they took 111, and a batch of few lasted as long as its longest unit: 40
+// requests of 1 to 100,000 queries on trees of 10,000 to 2M points 159 ms, now 38;
+// one query on 1M points 35.6 ms, now 0.18.
+template <int DIM, int K>
+__global__ void __launch_bounds__(kEvalThreads, 4)
+    batch_bf_kernel(BatchHeader* hdr, const BatchItem* __restrict__ items,
+                    const DevTree* __restrict__ trees, int warp_words, PlainSum* partial,
+                    unsigned* counters) {
+  extern __shared__ float4 s_eval[];
+  float* wbase = reinterpret_cast<float*>(s_eval) + (size_t)(threadIdx.x >> 5) * warp_words;
+  PlainSum* tot = reinterpret_cast<PlainSum*>(wbase + kTreeWords + kItemWords);
+  for_each_unit(hdr, items, trees, batch_class(0, DIM, K), wbase,
+                [&](const DevTree& t, const BatchItem& it, long long u) {
+                  run_bf<DIM, K>(t, it, u, tot, partial, counters);
+                });
+}
+
 // Per-warp shared words of a class's kernel for a launch shape: the tree and
 // request records, then the class's scratch (Barnes-Hut stack of `bh_stack`
-// entries, or sampler scratch for roots of up to `sbh_r` children).
-int class_warp_words(int cls, int bh_stack, int sbh_r) {
+// entries or bh_query_task's scratch, or sampler scratch for roots of up to `sbh_r` children).
+int class_warp_words(int cls, int bh_stack, bool bh_query, int sbh_r) {
   int scratch = 0;
   if (cls == kClassBh) scratch = bh_stack * (int)sizeof(BhStackEntry) / 4;
+  if (cls == kClassBh && bh_query)
+    scratch = std::max(scratch, (int)(bh_query_smem(bh_stack) / 4));
   if (cls == kClassSbh) scratch = sbh_warp_words<float>();
-  if (cls == kClassBf) scratch = (int)(32 * (sizeof(SrcPair) + sizeof(NrmPair)) / 4);
+  if (cls >= kClassBf) scratch = kBfTileQueries * (int)sizeof(PlainSum) / 4;
   (void)sbh_r;
   return kTreeWords + kItemWords + (scratch + 3) / 4 * 4;
 }
 
-size_t class_smem(int cls, int bh_stack, int sbh_r) {
-  return (size_t)kEvalWarps * class_warp_words(cls, bh_stack, sbh_r) * sizeof(float);
+size_t class_smem(int cls, int bh_stack, bool bh_query, int sbh_r) {
+  return (size_t)kEvalWarps * class_warp_words(cls, bh_stack, bh_query, sbh_r) * sizeof(float);
 }
 
-template <int CLASS>
-void allow_smem(size_t smem) {
+using BfKernel = void (*)(BatchHeader*, const BatchItem*, const DevTree*, int, PlainSum*, unsigned*);
+const BfKernel kBfKernels[8] = {
+    batch_bf_kernel<3, kGravity>,    batch_bf_kernel<3, kWindingNumber>,
+    batch_bf_kernel<3, kSmoothDist>, batch_bf_kernel<3, kPlummer>,
+    batch_bf_kernel<2, kGravity>,    batch_bf_kernel<2, kWindingNumber>,
+    batch_bf_kernel<2, kSmoothDist>, batch_bf_kernel<2, kPlummer>};
+
+const void* class_kernel(int cls) {
+  if (cls == kClassBh) return reinterpret_cast<const void*>(batch_eval_kernel<kClassBh>);
+  if (cls == kClassSbh) return reinterpret_cast<const void*>(batch_eval_kernel<kClassSbh>);
+  return reinterpret_cast<const void*>(kBfKernels[cls - kClassBf]);
+}
+
+void allow_smem(int cls, size_t smem) {
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(batch_eval_kernel<CLASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-}
-
-template <int CLASS>
-int occupancy(size_t smem) {
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_eval_kernel<CLASS>, kEvalThreads, smem);
-  return std::max(1, n);
+    cudaFuncSetAttribute(class_kernel(cls), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 int class_occupancy(int cls, size_t smem) {
-  return cls == kClassBh ? occupancy<kClassBh>(smem)
-         : cls == kClassSbh ? occupancy<kClassSbh>(smem)
-                            : occupancy<kClassBf>(smem);
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, class_kernel(cls), kEvalThreads, smem);
+  return std::max(1, n);
 }
 
 // Launch shapes are rounded so that few graphs serve every batch: the stack
@@ -354,6 +454,9 @@ int round_root(int need, const BatchEngine::Limits& lim) {
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// Tile parts a batch may split its brute force into (16 MiB of sums).
+constexpr long long kMaxTileParts = 1LL << 18;
 
 // Bucket capacity: at least 2 queries per bucket (the tuning's lower bound),
 // plus a bucket per request for requests below a full bucket.
@@ -381,7 +484,9 @@ BatchEngine::BatchEngine(const Limits& lim, int sm_count) : lim_(lim), sm_count_
   const size_t o_order = o_hist + align256(sizeof(unsigned) * nb);
   const size_t o_qbox = o_order + align256(sizeof(int) * lim_.max_queries);
   const size_t o_sums = o_qbox + align256(sizeof(unsigned) * 6 * lim_.max_items);
-  dev_bytes_ = o_sums + align256(sizeof(unsigned) * scan_tiles_for(nb));
+  const size_t o_partial = o_sums + align256(sizeof(unsigned) * scan_tiles_for(nb));
+  const size_t o_counters = o_partial + align256(sizeof(PlainSum) * kBfTileQueries * kMaxTileParts);
+  dev_bytes_ = o_counters + align256(sizeof(unsigned) * kMaxTileParts / 2);
   if (cudaMalloc(&dev_, dev_bytes_) != cudaSuccess) {
     dev_ = nullptr;
     return;
@@ -394,16 +499,18 @@ BatchEngine::BatchEngine(const Limits& lim, int sm_count) : lim_(lim), sm_count_
   d_order_ = reinterpret_cast<int*>(b + o_order);
   d_qbox_ = reinterpret_cast<unsigned*>(b + o_qbox);
   d_sums_ = reinterpret_cast<unsigned*>(b + o_sums);
+  d_partial_ = reinterpret_cast<PlainSum*>(b + o_partial);
+  d_counters_ = reinterpret_cast<unsigned*>(b + o_counters);
+  // at zero between batches: a tile's last unit puts its counter back
+  cudaMemset(d_counters_, 0, sizeof(unsigned) * kMaxTileParts / 2);
   if (cudaMallocHost(&h_stage_, o_keys) != cudaSuccess) h_stage_ = nullptr;
   // Allow each class's kernel the shared memory of the engine's largest
   // shape; report occupancy at the smallest (the register bound).
   const int big_stack = lim_.max_tree_depth + 2, big_root = lim_.max_root_children;
-  allow_smem<kClassBh>(class_smem(kClassBh, big_stack, big_root));
-  allow_smem<kClassSbh>(class_smem(kClassSbh, big_stack, big_root));
-  allow_smem<kClassBf>(class_smem(kClassBf, big_stack, big_root));
+  for (int c = 0; c < kClasses; c++) allow_smem(c, class_smem(c, big_stack, true, big_root));
   const int small_stack = round_stack(0, lim_), small_root = round_root(0, lim_);
   for (int c = 0; c < kClasses; c++)
-    per_sm_[c] = class_occupancy(c, class_smem(c, small_stack, small_root));
+    per_sm_[c] = class_occupancy(c, class_smem(c, small_stack, false, small_root));
 }
 
 BatchEngine::~BatchEngine() {
@@ -429,28 +536,53 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
   // sampler: sampled paths per query), so that the class's warps take the long
   // units early and the short ones fill in at the end.  The order changes no
   // result: every unit is summed by one warp on its own.
+  auto class_of = [&](const BatchItem& it) {
+    return batch_class(it.method, host_trees[it.tree].dim, it.kernel);
+  };
   auto unit_cost = [&](const BatchItem& it) -> double {
     const DevTree& t = host_trees[it.tree];
-    if (batch_class(it.method) == kClassBf) return (double)t.n;
-    if (batch_class(it.method) == kClassSbh) return (double)it.samples * t.root_children;
+    if (it.method == 0) return (double)t.n;
+    if (it.method == 3) return (double)it.samples * t.root_children;
     return 0.0;
   };
   std::stable_sort(items.begin(), items.end(), [&](const BatchItem& a, const BatchItem& b) {
-    const int ca = batch_class(a.method), cb = batch_class(b.method);
+    const int ca = class_of(a), cb = class_of(b);
     if (ca != cb) return ca < cb;
     return unit_cost(a) > unit_cost(b);
   });
-  long long sampled = 0;
-  for (const BatchItem& it : items)
-    if (batch_class(it.method) == kClassSbh) sampled += it.nq;
+  long long sampled = 0, walked = 0;
+  double bf_work = 0.0;  // sources read by all brute-force tiles
+  for (const BatchItem& it : items) {
+    if (it.method == 3) sampled += it.nq;
+    if (it.method == 1) walked += it.nq;
+    if (it.method == 0)
+      bf_work += (double)((it.nq + kBfTileQueries - 1) / kBfTileQueries) *
+                 (double)host_trees[it.tree].n;
+  }
+  // Barnes-Hut walks: a warp per query under the same rule as a single call,
+  // here by the batch's queries, and in larger batches for requests of up to
+  // kBhUnorderedQueries, whose neighbours share too little of a walk (40 requests
+  // of 1 to 100,000 queries, theta 0.2: 22.9 ms a lane per query throughout, 12.1
+  // with this); units of a few queries where there are many.
+  const bool all_per_query = bh_query_per_warp(walked, sm_count_);
+  int walk_unit = 1;
+  while (walk_unit < 8 && walked > 64LL * walk_unit * sm_count_) walk_unit *= 2;
+  // Brute force: a tile's sum over all sources is one unit while that is at most
+  // an eighth of a warp's share of the batch; longer ones are split into their
+  // parts (largest trees first, as far as the partial sums' room goes), since the
+  // batch ends with its longest unit.
+  const double bf_share = bf_work / ((double)per_sm_[kClassBf] * kEvalWarps * sm_count_);
+  long long tile_parts = 0, split_tiles = 0;
   const int sampler_unit = std::min(tuning.sampler_unit, sampler_group(sampled, sm_count_));
-  long long sort_base = 0, bucket_base = 0, unit_base[kClasses] = {0, 0, 0};
+  long long sort_base = 0, bucket_base = 0, unit_base[kClasses] = {};
   for (BatchItem& it : items) {
     if (it.tree < 0 || it.tree >= (int)host_trees.size()) return "request names an unknown tree";
     const DevTree& t = host_trees[it.tree];
     if (t.depth + 2 > lim_.max_tree_depth + 2) return "tree deeper than the engine supports";
     if (t.root_children > lim_.max_root_children) return "tree root wider than the engine supports";
-    const bool sorted = it.method == 1;  // vote and the sampler keep the caller's order
+    it.per_query = it.method == 1 && (all_per_query || it.nq <= kBhUnorderedQueries);
+    // vote and the sampler keep the caller's order, and so do few walks
+    const bool sorted = it.method == 1 && !(it.per_query && it.nq <= kBhUnorderedQueries);
     it.sort_bits =
         (sorted && it.sort_bits >= 0) ? sort_bits_for(it.nq, t.dim, tuning.bucket_queries) : 0;
     it.dim = t.dim;
@@ -459,19 +591,32 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
     it.sort_base = sort_base;
     it.bucket_base = bucket_base;
     it.buckets = it.sort_bits > 0 ? (1LL << (t.dim * it.sort_bits)) : 1;
-    it.unit_base = unit_base[batch_class(it.method)];
+    it.unit_base = unit_base[class_of(it)];
     // Work unit: sampler queries per warp (tuned; fewer in batches of few, as in
     // a single call); Barnes-Hut queries per warp
     // walk (tuned; vote keeps 32, its acceptance is defined over 32 queries);
-    // brute force kBfUnitQueries per warp (query pairs per lane, tasks.cuh).
+    // brute force kBfTileQueries per warp against all sources or a part of them.
     it.unit_queries = it.method == 3   ? sampler_unit
-                      : it.method == 1 ? tuning.bh_unit
-                      : it.method == 0 ? kBfUnitQueries
+                      : it.method == 1 ? (it.per_query ? walk_unit : tuning.bh_unit)
+                      : it.method == 0 ? kBfTileQueries
                                        : kUnitQueriesWarp;
     it.units = (it.nq + it.unit_queries - 1) / it.unit_queries;
+    it.split = 0;
+    if (it.method == 0) {
+      const int parts = bf_parts(t.n);
+      if (parts > 1 && (double)t.n > bf_share / 8 &&
+          tile_parts + it.units * parts <= kMaxTileParts) {
+        it.split = parts;
+        it.partial_base = tile_parts * kBfTileQueries;
+        it.counter_base = split_tiles;
+        tile_parts += it.units * parts;
+        split_tiles += it.units;
+        it.units *= parts;
+      }
+    }
     sort_base += it.nq;
     bucket_base += it.buckets;
-    unit_base[batch_class(it.method)] += it.units;
+    unit_base[class_of(it)] += it.units;
   }
   if (sort_base > lim_.max_queries) return "batch exceeds the engine's query capacity";
   if (bucket_base > max_buckets(lim_)) return "batch exceeds the engine's bucket capacity";
@@ -507,13 +652,14 @@ cudaError_t BatchEngine::capture(const DevTree* d_trees, int* d_status, const Sh
                                                                 d_hist_, d_order_);
     cudaEventRecord(ev[0], st[0]);
     for (int c = 0; c < kClasses; c++) {
+      if (!((shape.classes >> c) & 1u)) continue;
       cudaStream_t s = c == 0 ? st[0] : st[c];
       if (c > 0) cudaStreamWaitEvent(s, ev[0], 0);
-      const size_t smem = class_smem(c, shape.bh_stack, shape.sbh_root);
+      const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
       const int fit = class_occupancy(c, smem);
       const int per_sm = shape.per_sm_cap > 0 ? std::min(shape.per_sm_cap, fit) : fit;
       const int blocks = per_sm * sm_count_;
-      const int words = class_warp_words(c, shape.bh_stack, shape.sbh_root);
+      const int words = class_warp_words(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
       if (c == kClassBh)
         batch_eval_kernel<kClassBh><<<blocks, kEvalThreads, smem, s>>>(
             d_header_, d_items_, d_trees, d_order_, d_status, words, stack_cap);
@@ -521,8 +667,8 @@ cudaError_t BatchEngine::capture(const DevTree* d_trees, int* d_status, const Sh
         batch_eval_kernel<kClassSbh><<<blocks, kEvalThreads, smem, s>>>(
             d_header_, d_items_, d_trees, d_order_, d_status, words, stack_cap);
       else
-        batch_eval_kernel<kClassBf><<<blocks, kEvalThreads, smem, s>>>(
-            d_header_, d_items_, d_trees, d_order_, d_status, words, stack_cap);
+        kBfKernels[c - kClassBf]<<<blocks, kEvalThreads, smem, s>>>(
+            d_header_, d_items_, d_trees, words, d_partial_, d_counters_);
       if (c > 0) {
         cudaEventRecord(ev[c], s);
         cudaStreamWaitEvent(st[0], ev[c], 0);
@@ -556,7 +702,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   }
   int need_depth = 0, need_root = 0;
   for (const BatchItem& it : items) {
-    const int c = batch_class(it.method);
+    const int c = batch_class(it.method, it.dim, it.kernel);
     if (c == kClassBh) need_depth = std::max(need_depth, it.depth);
     if (c == kClassSbh) need_root = std::max(need_root, it.root_children);
   }
@@ -564,10 +710,19 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   shape.per_sm_cap = std::max(0, tuning.blocks_per_sm);
   shape.bh_stack = round_stack(need_depth + 2, lim_);
   shape.sbh_root = round_root(need_root, lim_);
+  for (const BatchItem& it : items) {
+    shape.bh_query = shape.bh_query || it.per_query;
+    shape.classes |= 1u << batch_class(it.method, it.dim, it.kernel);
+  }
   cudaGraphExec_t exec = nullptr;
   for (const Graph& g : graphs_)
     if (g.shape == shape) exec = g.exec;
   if (!exec) {
+    if (graphs_.size() >= 32) {  // shapes are few; never let them pile up
+      for (Graph& g : graphs_)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+      graphs_.clear();
+    }
     cudaError_t e = capture(d_trees, d_status, shape, &exec);
     if (e != cudaSuccess) return e;
     graphs_.push_back(Graph{shape, exec});
@@ -578,7 +733,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   int prev = -1;
   for (int i = 0; i < (int)items.size(); i++) {
     const BatchItem& it = items[i];
-    const int c = batch_class(it.method);
+    const int c = batch_class(it.method, it.dim, it.kernel);
     if (c != prev) {
       h.item_begin[c] = i;
       prev = c;

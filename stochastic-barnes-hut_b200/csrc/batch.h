@@ -13,6 +13,8 @@
 
 namespace sbh {
 
+struct PlainSum;  // a compensated sum (lane_sum.cuh)
+
 // One request of a batch, as the device reads it.
 struct BatchItem {
   int tree;                  // index into the engine's tree table
@@ -39,14 +41,22 @@ struct BatchItem {
   long long buckets;         // buckets of this request
   long long unit_base;       // first work unit of this request within its class
   long long units;           // work units of this request
+  int per_query;             // Barnes-Hut: a warp per query (bh_query_task)
+  int split;                 // brute force: parts per tile that are units of their own
+                             // (0: a unit sums all parts)
+  long long partial_base;    // first tile sum of a split request's parts
+  long long counter_base;    // first tile counter of a split request
 };
 
-// Requests are evaluated by one persistent kernel per method class (each
-// compiled for its own method, so none pays for the others' registers):
-enum BatchClass : int { kClassBh = 0, kClassSbh = 1, kClassBf = 2, kClasses = 3 };
+// Requests are evaluated by one persistent kernel per class, each compiled for
+// its own work alone, so none pays for another's registers: Barnes-Hut, the
+// sampler, and brute force by dimension and kernel function.
+enum BatchClass : int { kClassBh = 0, kClassSbh = 1, kClassBf = 2, kClasses = 2 + 8 };
 
-__host__ __device__ inline int batch_class(int method) {
-  return method == 3 ? kClassSbh : (method == 1 || method == 2) ? kClassBh : kClassBf;
+__host__ __device__ inline int batch_class(int method, int dim, int kernel) {
+  return method == 3 ? kClassSbh
+         : (method == 1 || method == 2) ? kClassBh
+                                        : kClassBf + (dim == 3 ? 0 : 4) + kernel;
 }
 
 struct BatchHeader {
@@ -60,8 +70,8 @@ struct BatchHeader {
 };
 
 // Queries per work unit (one warp task) of warp-vote Barnes-Hut: 32, a lane
-// each (brute force takes kBfUnitQueries, 2 x kBfUnitPairs per lane).  The sampler's and
-// Barnes-Hut's unit sizes (queries per warp task) are tuned.
+// each (brute force takes kBfTileQueries).  The sampler's and Barnes-Hut's unit
+// sizes (queries per warp task) are tuned.
 constexpr int kUnitQueriesWarp = 32;
 
 class BatchEngine {
@@ -108,7 +118,7 @@ class BatchEngine {
   // CTAs per SM of the evaluation kernels at full occupancy (the largest, at
   // the smallest launch shape).
   int max_blocks_per_sm() const {
-    return std::max(per_sm_[0], std::max(per_sm_[1], per_sm_[2]));
+    return *std::max_element(per_sm_, per_sm_ + kClasses);
   }
 
  private:
@@ -116,9 +126,12 @@ class BatchEngine {
   struct Shape {
     int per_sm_cap = 0;  // the tuning's CTAs-per-SM cap (0: none)
     int bh_stack = 0;    // Barnes-Hut stack entries per warp
+    bool bh_query = false;  // whether the scratch holds bh_query_task's
     int sbh_root = 0;    // widest sampler root the scratch holds
+    unsigned classes = 0;  // bit c: the batch has requests of class c
     bool operator==(const Shape& o) const {
-      return per_sm_cap == o.per_sm_cap && bh_stack == o.bh_stack && sbh_root == o.sbh_root;
+      return per_sm_cap == o.per_sm_cap && bh_stack == o.bh_stack && bh_query == o.bh_query &&
+             sbh_root == o.sbh_root && classes == o.classes;
     }
   };
   struct Graph {
@@ -130,7 +143,7 @@ class BatchEngine {
 
   Limits lim_;
   int sm_count_;
-  int per_sm_[kClasses] = {1, 1, 1};  // at the smallest launch shape
+  int per_sm_[kClasses] = {};  // at the smallest launch shape
   // device buffers
   void* dev_ = nullptr;
   size_t dev_bytes_ = 0;
@@ -141,6 +154,8 @@ class BatchEngine {
   int* d_order_ = nullptr;
   unsigned* d_qbox_ = nullptr;  // per request: its queries' bounding box
   unsigned* d_sums_ = nullptr;  // tile sums of the bucket scan
+  PlainSum* d_partial_ = nullptr;  // split brute force: the tiles' sums, part by part ...
+  unsigned* d_counters_ = nullptr;  // ... and how many of a tile's parts are done
   // pinned staging of header + items
   void* h_stage_ = nullptr;
   // captured pipelines, one per launch shape

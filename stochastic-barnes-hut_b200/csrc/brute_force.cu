@@ -25,85 +25,6 @@
 namespace sbh {
 namespace {
 
-// A lane's compensated sum of one query.
-struct PlainSum {
-  float hi, lo;
-  __device__ __forceinline__ void merge(const PlainSum& b) {
-    two_sum_add(hi, lo, b.hi);
-    lo += b.lo;
-  }
-};
-
-// A lane's NP query pairs (split_sum.cuh).
-template <int DIM, int K, int NP>
-struct PlainAcc {
-  using Sum = PlainSum;
-  static constexpr int Q = 2 * NP;
-  static constexpr int kMinCtas = NP == 4 ? 2 : K == kWindingNumber ? 3 : 4;  // no spills
-  static constexpr bool kNormals = K == kWindingNumber;
-  float2 nqx[NP], nqy[NP], nqz[NP], part[NP];
-  float hi[Q], lo[Q];
-  KParams kp;
-
-  __device__ __forceinline__ void load(const float* qsoa, long long nq, long long q0,
-                                       const KParams& params) {
-    kp = params;
-#pragma unroll
-    for (int p = 0; p < NP; p++) {
-      float3 a = make_float3(0.f, 0.f, 0.f), b = a;
-      if (q0 + 2 * p < nq) a = load_query<DIM>(qsoa, nq, q0 + 2 * p);
-      if (q0 + 2 * p + 1 < nq) b = load_query<DIM>(qsoa, nq, q0 + 2 * p + 1);
-      nqx[p] = make_float2(-a.x, -b.x);
-      nqy[p] = make_float2(-a.y, -b.y);
-      nqz[p] = make_float2(-a.z, -b.z);
-      part[p] = make_float2(0.f, 0.f);
-      hi[2 * p] = lo[2 * p] = hi[2 * p + 1] = lo[2 * p + 1] = 0.f;
-    }
-  }
-  template <int MODE>
-  __device__ __forceinline__ void add(float4 s, float4 n) {
-    const SrcPair sp = {dup(s.x), dup(s.y), dup(s.z), dup(s.w)};
-    const NrmPair np = {dup(n.x), dup(n.y), dup(n.z), dup(0.f)};
-#pragma unroll
-    for (int p = 0; p < NP; p++)
-      part[p] = accumulate2<DIM, K, MODE>(part[p], sp, np, nqx[p], nqy[p], nqz[p], kp);
-  }
-  __device__ __forceinline__ bool scaled() const { return K == kSmoothDist && kp.alpha >= 0.f; }
-  __device__ __forceinline__ void group(const float4 (&s)[kSplitGroup],
-                                        const float4 (&n)[kSplitGroup]) {
-    static_assert(kSplitGroup == kSdFmaEvery, "one source of a group on the FP32 pipe");
-    if (scaled()) {
-      add<2>(s[0], n[0]);
-#pragma unroll
-      for (int i = 1; i < kSplitGroup; i++) add<1>(s[i], n[i]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < kSplitGroup; i++) add<0>(s[i], n[i]);
-    }
-  }
-  __device__ __forceinline__ void single(float4 s, float4 n) {
-    if (scaled())
-      add<1>(s, n);
-    else
-      add<0>(s, n);
-  }
-  __device__ __forceinline__ void flush() {
-#pragma unroll
-    for (int p = 0; p < NP; p++) {
-      if (scaled()) part[p] = __fmul2_rn(part[p], dup(kExp2Unscale));
-      two_sum_add(hi[2 * p], lo[2 * p], part[p].x);
-      two_sum_add(hi[2 * p + 1], lo[2 * p + 1], part[p].y);
-      part[p] = make_float2(0.f, 0.f);
-    }
-  }
-  __device__ __forceinline__ Sum sum(int j) const { return Sum{hi[j], lo[j]}; }
-  __device__ __forceinline__ static void store(float* out, float*, long long, long long qi,
-                                               const Sum& s, const KParams&) {
-    const float v = s.hi + s.lo;
-    out[qi] = K == kGravity ? -v : v;
-  }
-};
-
 template <int DIM, int K>
 cudaError_t launch_bf(const DevTree& t, const float* q, long long nq, const KParams& kp, float* out,
                       cudaStream_t stream, int sm_count) {

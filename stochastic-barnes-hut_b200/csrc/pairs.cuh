@@ -1,8 +1,6 @@
 // Packed FP32x2 kernel arithmetic of the all-pairs summations: two queries per
 // instruction on Blackwell's FADD2 / FMUL2 / FFMA2, sources held with every
-// coordinate duplicated into both halves of a float2 (shared by the single-call
-// brute-force kernel, brute_force.cu, and the batched brute-force task,
-// tasks.cuh).
+// coordinate duplicated into both halves of a float2 (lane_sum.cuh, adjoint.cu).
 #pragma once
 
 #include "device_common.cuh"
@@ -16,6 +14,15 @@ struct __align__(16) SrcPair {
 struct __align__(16) NrmPair {
   float2 x, y, z, unused;
 };
+
+// Knuth two-sum of (hi, lo) += s.
+__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float s) {
+  const float t = hi + s;
+  const float bp = t - hi;
+  const float e = (hi - (t - bp)) + (s - bp);
+  hi = t;
+  lo += e;
+}
 
 __device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
 
@@ -153,50 +160,6 @@ __device__ __forceinline__ float2 accumulate2(float2 part, const SrcPair& s, con
     }
     const float2 t = __fmul2_rn(dup(-kp.alpha * 1.44269504088896341f), norm_from_sq(r2));
     return __fadd2_rn(part, make_float2(mufu_ex2(t.x), mufu_ex2(t.y)));
-  }
-}
-
-// part[p] += the smooth-distance values of the staged sources 0 .. n-1 (N > 0:
-// n = N, known at compile time) at query pair p; src(k) returns staged source
-// k (an accessor, so that a caller indexing a __shared__ array keeps its
-// shared-memory loads).  alpha >= 0 takes the scaled form, one source in
-// kSdFmaEvery on the FP32 pipe, and unscales the sums at the end; alpha < 0
-// (powers beyond the scaled range) takes the plain form.
-template <int DIM, int NP, int N, class Src>
-__device__ __forceinline__ void accumulate_smooth(float2 (&part)[NP], const Src& src, int n,
-                                                  const float2 (&nqx)[NP], const float2 (&nqy)[NP],
-                                                  const float2 (&nqz)[NP], const KParams& kp) {
-  constexpr int K = kSmoothDist;
-  const NrmPair none = {};
-  const int count = N > 0 ? N : n;
-  if (kp.alpha >= 0.f) {
-    int k = 0;
-#pragma unroll 1
-    for (; k + kSdFmaEvery <= count; k += kSdFmaEvery) {
-#pragma unroll
-      for (int i = 0; i < kSdFmaEvery; i++) {
-        const SrcPair s = src(k + i);
-#pragma unroll
-        for (int p = 0; p < NP; p++)
-          part[p] = i == 0 ? accumulate2<DIM, K, 2>(part[p], s, none, nqx[p], nqy[p], nqz[p], kp)
-                           : accumulate2<DIM, K, 1>(part[p], s, none, nqx[p], nqy[p], nqz[p], kp);
-      }
-    }
-    for (; k < count; k++) {
-      const SrcPair s = src(k);
-#pragma unroll
-      for (int p = 0; p < NP; p++)
-        part[p] = accumulate2<DIM, K, 1>(part[p], s, none, nqx[p], nqy[p], nqz[p], kp);
-    }
-#pragma unroll
-    for (int p = 0; p < NP; p++) part[p] = __fmul2_rn(part[p], dup(kExp2Unscale));
-  } else {
-    for (int k = 0; k < count; k++) {
-      const SrcPair s = src(k);
-#pragma unroll
-      for (int p = 0; p < NP; p++)
-        part[p] = accumulate2<DIM, K>(part[p], s, none, nqx[p], nqy[p], nqz[p], kp);
-    }
   }
 }
 

@@ -6,9 +6,8 @@
 // to keep a warp busy.  What is left of the parallelism goes over the sources:
 // `sw` of a CTA's 8 warps take parts of the sources of the same queries (the
 // others have queries of their own and read the same sources through L1), and a
-// cluster of up to 16 CTAs splits them further.  Every lane sums plain FP32 runs
-// of kSplitRun sources and merges each into a compensated sum; lanes, warps and CTAs
-// (through distributed shared memory, in rank order) merge those.  No scratch
+// cluster of up to 16 CTAs splits them further.  Lanes, warps and CTAs (through
+// distributed shared memory, in rank order) merge their compensated sums.  No scratch
 // memory, one launch, and the result depends only on the call's shape.
 #pragma once
 
@@ -16,29 +15,14 @@
 
 #include <algorithm>
 
-#include "device_common.cuh"
+#include "lane_sum.cuh"
 
 namespace sbh {
 namespace {
 
 constexpr int kSplitWarps = 8;
 constexpr int kSplitThreads = 32 * kSplitWarps;
-constexpr int kSplitGroup = 4;  // sources a lane loads at a time
-constexpr int kSplitRun = 32;   // sources of a plain FP32 sum
-
-template <class T>
-__device__ __forceinline__ T shfl_down_words(const T& v, int d) {
-  static_assert(sizeof(T) % 4 == 0, "word-sized members");
-  T r;
-  const int* src = reinterpret_cast<const int*>(&v);
-  int* dst = reinterpret_cast<int*>(&r);
-#pragma unroll
-  for (int w = 0; w < (int)(sizeof(T) / 4); w++) dst[w] = __shfl_down_sync(0xffffffffu, src[w], d);
-  return r;
-}
-
-// Acc: a lane's state for Q queries.  load() reads them, group() adds
-// kSplitGroup sources, single() one, flush() ends a run, sum(j) is query j's
+// Acc: a lane's state for Q queries (lane_sum.cuh); sum(j) is query j's
 // compensated sum (Acc::Sum, with merge()), store() writes a query's result.
 template <class Acc, int DIM>
 __global__ void __launch_bounds__(kSplitThreads, Acc::kMinCtas)
@@ -63,41 +47,11 @@ __global__ void __launch_bounds__(kSplitThreads, Acc::kMinCtas)
 
   Acc acc;
   acc.load(qsoa, nq, (tile0 + warp / sw) * Q, kp);
-  // The next group is loaded before the current one is summed.
-  const long long full_end = c0 + (c1 - c0) / (32 * kSplitGroup) * (32 * kSplitGroup);
-  long long base = c0;
-  float4 s[kSplitGroup], nr[kSplitGroup], s2[kSplitGroup], nr2[kSplitGroup];
-  auto fetch = [&](long long at, float4 (&s)[kSplitGroup], float4 (&nr)[kSplitGroup]) {
-#pragma unroll
-    for (int i = 0; i < kSplitGroup; i++) {
-      s[i] = __ldg(t.pt_pm + at + 32 * i + lane);
-      nr[i] = Acc::kNormals ? __ldg(t.pt_nrm + at + 32 * i + lane)
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  if (base < full_end) fetch(base, s, nr);
-  int run = 0;
-  for (; base < full_end; base += 32 * kSplitGroup) {
-    const bool more = base + 32 * kSplitGroup < full_end;
-    if (more) fetch(base + 32 * kSplitGroup, s2, nr2);
-    acc.group(s, nr);
-    if ((++run & (kSplitRun / kSplitGroup - 1)) == 0) acc.flush();
-#pragma unroll
-    for (int i = 0; i < kSplitGroup; i++) {
-      s[i] = s2[i];
-      nr[i] = nr2[i];
-    }
-  }
-  for (base += lane; base < c1; base += 32)
-    acc.single(__ldg(t.pt_pm + base), Acc::kNormals ? __ldg(t.pt_nrm + base)
-                                                    : make_float4(0.f, 0.f, 0.f, 0.f));
-  acc.flush();
+  sum_range(acc, t.pt_pm, t.pt_nrm, c0, c1);
 
 #pragma unroll
   for (int j = 0; j < Q; j++) {
-    Sum v = acc.sum(j);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v.merge(shfl_down_words(v, o));
+    const Sum v = merge_lanes(acc.sum(j));
     if (lane == 0) s_warp[warp * Q + j] = v;
   }
   __syncthreads();

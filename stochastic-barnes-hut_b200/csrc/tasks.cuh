@@ -4,6 +4,7 @@
 #pragma once
 
 #include "device_common.cuh"
+#include "lane_sum.cuh"
 #include "pairs.cuh"
 #include "sums.cuh"
 
@@ -1005,108 +1006,21 @@ __device__ __forceinline__ void sbh_warp_task(
 
 // ======================================================= brute force ===
 
-// Knuth two-sum of (hi, lo) += s.
-__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float s) {
-  const float t = hi + s;
-  const float bp = t - hi;
-  const float e = (hi - (t - bp)) + (s - bp);
-  hi = t;
-  lo += e;
+// The batched brute-force task's queries per warp.
+constexpr int kBfTileQueries = 8;
+
+// Sources of one part of a tree of n: its sums are merged in part order, so a
+// request's results do not depend on whether one warp sums all parts of a tile of
+// queries or each part is a work unit of its own.  16,384 sources (merging the
+// lanes' sums takes 1.5% of that), or as many as make 128 parts.
+__host__ __device__ inline long long bf_part_sources(long long n) {
+  const long long most = (n + 127) / 128;
+  return most > 16384 ? (most + 31) / 32 * 32 : 16384;
 }
-
-// Query pairs per lane of the batched brute-force task, and its queries per
-// work unit (a warp's 32 lanes x two queries per pair).  Two pairs per lane
-// (176 registers, fewer warps per SM) measured 15% slower than one on B200.
-constexpr int kBfUnitPairs = 1;
-constexpr int kBfUnitQueries = 64 * kBfUnitPairs;
-
-// Brute force for up to kBfUnitQueries queries at positions [slot0, slot_end)
-// of a request, one warp: the batch's brute-force task.  Lane l holds queries
-// slot0 + l + 32 j (j < 2 kBfUnitPairs) as packed pairs (j = 2p, 2p + 1): the
-// single-call kernel's FP32x2 arithmetic (pairs.cuh).  The warp stages 32
-// sources at a time in its shared memory (src / nrm, 32 entries each) with every
-// coordinate duplicated into both halves of a float2, and every lane reads them
-// back as broadcasts.  Plain FP32 sums over each 32 sources, merged into a
-// (sum, error) pair per query by two-sum.
-template <int DIM, int K>
-__device__ __forceinline__ void bf_warp_task(const DevTree& t, const float* __restrict__ qsoa,
-                                             long long nq, long long slot0, long long slot_end,
-                                             const KParams& kp, float* __restrict__ out,
-                                             int* __restrict__ contribs,
-                                             const float* __restrict__ self_mass, SrcPair* src,
-                                             NrmPair* nrm) {
-  constexpr bool kNormals = (K == kWindingNumber);
-  constexpr int NP = kBfUnitPairs;
-  const int lane = threadIdx.x & 31;
-  float2 nqx[NP], nqy[NP], nqz[NP];
-  float hi[2 * NP], lo[2 * NP];
-  const NrmPair no_normal = {};
-#pragma unroll
-  for (int p = 0; p < NP; p++) {
-    const long long qa = slot0 + 64 * p + lane, qb = qa + 32;
-    float3 a = make_float3(0.f, 0.f, 0.f), b = a;
-    if (qa < slot_end) a = load_query<DIM>(qsoa, nq, qa);
-    if (qb < slot_end) b = load_query<DIM>(qsoa, nq, qb);
-    nqx[p] = make_float2(-a.x, -b.x);
-    nqy[p] = make_float2(-a.y, -b.y);
-    nqz[p] = make_float2(-a.z, -b.z);
-    hi[2 * p] = lo[2 * p] = hi[2 * p + 1] = lo[2 * p + 1] = 0.f;
-  }
-  for (long long base = 0; base < t.n; base += 32) {
-    const int len = (int)min(32LL, t.n - base);
-    __syncwarp();  // every lane is done with the previous sources
-    if (lane < len) {
-      const float4 v = __ldg(t.pt_pm + base + lane);
-      src[lane] = SrcPair{dup(v.x), dup(v.y), dup(v.z), dup(v.w)};
-      if (kNormals) {
-        const float4 n = __ldg(t.pt_nrm + base + lane);
-        nrm[lane] = NrmPair{dup(n.x), dup(n.y), dup(n.z), dup(0.f)};
-      }
-    }
-    __syncwarp();
-    float2 part[NP];
-#pragma unroll
-    for (int p = 0; p < NP; p++) part[p] = make_float2(0.f, 0.f);
-    if (K == kSmoothDist) {
-      // its exponential split between the MUFU and the FP32 pipe (pairs.cuh)
-      const auto srck = [&](int k) { return src[k]; };
-      if (len == 32)
-        accumulate_smooth<DIM, NP, 32>(part, srck, 32, nqx, nqy, nqz, kp);
-      else
-        accumulate_smooth<DIM, NP, 0>(part, srck, len, nqx, nqy, nqz, kp);
-    } else if (len == 32) {
-#pragma unroll 8
-      for (int k = 0; k < 32; k++) {
-        const NrmPair nr = kNormals ? nrm[k] : no_normal;
-#pragma unroll
-        for (int p = 0; p < NP; p++)
-          part[p] = accumulate2<DIM, K>(part[p], src[k], nr, nqx[p], nqy[p], nqz[p], kp);
-      }
-    } else {
-      for (int k = 0; k < len; k++) {
-        const NrmPair nr = kNormals ? nrm[k] : no_normal;
-#pragma unroll
-        for (int p = 0; p < NP; p++)
-          part[p] = accumulate2<DIM, K>(part[p], src[k], nr, nqx[p], nqy[p], nqz[p], kp);
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < NP; p++) {
-      two_sum_add(hi[2 * p], lo[2 * p], part[p].x);
-      two_sum_add(hi[2 * p + 1], lo[2 * p + 1], part[p].y);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 2 * NP; j++) {
-    const long long qi = slot0 + 32 * j + lane;
-    if (qi < slot_end) {
-      float v = hi[j] + lo[j];
-      if (K == kGravity) v = -v;  // accumulate2 adds +m / (r + 0.1)
-      if (self_mass) v -= self_term<DIM, K>(load_query<DIM>(qsoa, nq, qi), __ldg(self_mass + qi), kp);
-      out[qi] = v;
-      if (contribs) contribs[qi] = (int)t.n;
-    }
-  }
+__host__ __device__ inline int bf_parts(long long n) {
+  const long long len = bf_part_sources(n);
+  const long long parts = (n + len - 1) / len;
+  return parts > 1 ? (int)parts : 1;
 }
 
 }  // namespace sbh
