@@ -12,10 +12,11 @@ namespace sbh {
 
 // ============================================================ Barnes-Hut ===
 
-struct BhStackEntry {
+struct __align__(16) BhStackEntry {
   int cur;        // next sibling to visit
   int end;        // one past the last sibling
   unsigned mask;  // lanes that visit this sibling range
+  int pad;        // one 16-byte access each way
 };
 
 // A warp's shared-memory buffer for the points of an accepted leaf, filled by
@@ -37,8 +38,8 @@ __device__ __forceinline__ typename A::V self_term(float3 q, float m, const KPar
 // One warp evaluates the queries at sorted positions [slot0, slot_end) (at
 // most 32, one per lane) by a single depth-first walk of the union of the
 // lanes' opened sets.  The walk keeps, per tree level, a range of sibling nodes
-// still to visit and the mask of lanes that reach them (`stk`, stack_cap >=
-// tree depth + 2 entries).  At each node every lane in the mask applies the
+// still to visit and the mask of lanes that reach them (the level in hand in
+// registers, those above it in `stk`, stack_cap >= tree depth + 2 entries).  At each node every lane in the mask applies the
 // reference's opening test (farFieldRatio >= beta, include/tree3d.h:134-153)
 // itself; lanes that accept add the node's aggregate (or its leaf points), the
 // others are passed on to the children.  So every lane visits exactly the nodes
@@ -77,38 +78,28 @@ __device__ __forceinline__ void bh_warp_task(const DevTree& t, const float* __re
   typename A::V total = A::zero();
   int nc = 0;
   uint32_t phase = 0;  // STAGE: parity of the stage barrier's current phase
-  if (lane == 0) {
-    stk[0] = BhStackEntry{0, 1, active};
-    if (STAGE) mbar_init(&stage->bar, 1);
-  }
-  __syncwarp();
-  int sp = 1;
-  long long budget = t.nn + 1;  // a walk visits each node at most once
-  while (sp > 0) {
+  if (STAGE && lane == 0) mbar_init(&stage->bar, 1);
+  if (STAGE) __syncwarp();
+  // The sibling range in hand stays in registers; the stack holds what is left
+  // of the ranges above it.
+  int cur = 0, end = 1, sp = 0;
+  unsigned mask = active;
+  const bool leaf_far = __int_as_float(0x7f800000) >= beta;  // a leaf's ratio is infinite
+  int budget = (int)min(t.nn + 1, 0x7fffffffLL);  // a walk visits each node at most once
+  for (;;) {
     if (--budget < 0) {
       if (lane == 0) report_status(status, kStatusTraversalLimit);
       break;
     }
-    const BhStackEntry e = stk[sp - 1];
-    __syncwarp();
-    const int node = e.cur;
-    if (e.cur + 1 == e.end) {
-      sp--;
-    } else if (lane == 0) {
-      stk[sp - 1].cur = e.cur + 1;
-    }
-    const bool in = (e.mask >> lane) & 1u;
+    const int node = cur;
+    const bool in = (mask >> lane) & 1u;
     // Topology and node record in one round trip (a one-point leaf's record is
     // its point).
     const int4 topo = __ldg(t.nd_topo + node);
     const float4 cm = __ldg(t.nd_cm + node);
+    const float4 ag = __ldg(t.nd_agg + node);
     const bool leaf = topo.y == 0;
-    bool acc = false;
-    if (leaf) {
-      acc = in && (__int_as_float(0x7f800000) >= beta);
-    } else if (in) {
-      acc = far_enough<DIM>(cm, q, beta);
-    }
+    bool acc = in && (leaf ? leaf_far : far_enough<DIM>(cm, q, beta));
     if (VOTE) {
       const unsigned rej = __ballot_sync(0xffffffffu, in && !acc);
       acc = in && rej == 0u;
@@ -148,20 +139,33 @@ __device__ __forceinline__ void bh_warp_task(const DevTree& t, const float* __re
           nc++;
         }
       } else {
-        total = A::add(total, A::node(cm, __ldg(t.nd_agg + node), q, kp));
+        total = A::add(total, A::node(cm, ag, q, kp));
         nc++;
       }
     }
     const unsigned open = __ballot_sync(0xffffffffu, in && !acc);
+    cur++;
     if (open != 0u && !leaf) {
-      if (sp >= stack_cap) {
-        if (lane == 0) report_status(status, kStatusStackOverflow);
-        break;
+      if (cur < end) {
+        if (sp >= stack_cap) {
+          if (lane == 0) report_status(status, kStatusStackOverflow);
+          break;
+        }
+        if (lane == 0) stk[sp] = BhStackEntry{cur, end, mask, 0};
+        sp++;
       }
-      if (lane == 0) stk[sp] = BhStackEntry{topo.x, topo.x + topo.y, open};
-      sp++;
+      cur = topo.x;
+      end = topo.x + topo.y;
+      mask = open;
+    } else if (cur == end) {
+      if (sp == 0) break;
+      __syncwarp();  // lane 0's entry is in place
+      const BhStackEntry e = stk[--sp];
+      __syncwarp();  // and read before it is overwritten
+      cur = e.cur;
+      end = e.end;
+      mask = e.mask;
     }
-    __syncwarp();
   }
   if (valid) {
     if (self_mass) total = A::sub(total, self_term<DIM, K, A>(q, __ldg(self_mass + qi), kp));
