@@ -49,28 +49,39 @@ __global__ void init_kernel(unsigned* box, unsigned* hist) {
   for (int k = i; k < kBuckets; k += gridDim.x * blockDim.x) hist[k] = 0u;
 }
 
-__global__ void bbox_kernel(const float* __restrict__ q, long long nq, int dim, unsigned* box) {
-  unsigned mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
+// The queries' box: warps, then the block, reduce before one block's six atomics
+// (4M queries: 149 us with six atomics a warp of 4,096 blocks).
+__global__ void __launch_bounds__(256)
+    bbox_kernel(const float* __restrict__ q, long long nq, int dim, unsigned* box) {
+  __shared__ unsigned s_box[8][6];
+  unsigned v[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nq;
        i += (long long)gridDim.x * blockDim.x) {
-    for (int d = 0; d < dim; d++) {
-      const float v = q[d * nq + i];
-      if (v == v) {  // NaN queries do not widen the box
-        const unsigned o = float_to_ordered(v);
-        mn[d] = min(mn[d], o);
-        mx[d] = max(mx[d], o);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float x = d < dim ? q[d * nq + i] : __int_as_float(0x7fc00000);
+      if (x == x) {  // NaN queries do not widen the box
+        const unsigned o = float_to_ordered(x);
+        v[d] = min(v[d], o);
+        v[3 + d] = max(v[3 + d], o);
       }
     }
   }
-  for (int d = 0; d < dim; d++) {
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-      mx[d] = max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(box + d, mn[d]);
-      atomicMax(box + 3 + d, mx[d]);
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const unsigned r = k < 3 ? __reduce_min_sync(0xffffffffu, v[k]) : __reduce_max_sync(0xffffffffu, v[k]);
+    if (lane == 0) s_box[warp][k] = r;
+  }
+  __syncthreads();
+  const int k = threadIdx.x;
+  if (k < 2 * 3 && k % 3 < dim) {
+    unsigned r = s_box[0][k];
+    for (int w = 1; w < 8; w++) r = k < 3 ? min(r, s_box[w][k]) : max(r, s_box[w][k]);
+    if (k < 3)
+      atomicMin(box + k, r);
+    else
+      atomicMax(box + k, r);
   }
 }
 
@@ -139,7 +150,7 @@ cudaError_t launch_query_sort(const float* q, long long nq, int dim, void* ws, i
   const int threads = 256;
   const unsigned grid = (unsigned)min((nq + threads - 1) / threads, 4096LL);
   init_kernel<<<256, 256, 0, stream>>>(w.box, w.hist);
-  bbox_kernel<<<grid, threads, 0, stream>>>(q, nq, dim, w.box);
+  bbox_kernel<<<min(grid, 1184u), threads, 0, stream>>>(q, nq, dim, w.box);
   key_kernel<<<grid, threads, 0, stream>>>(q, nq, dim, w.box, w.keys, w.hist);
   launch_scan(w.hist, nullptr, kBuckets, kBuckets, w.sums, stream);
   scatter_kernel<<<grid, threads, 0, stream>>>(w.keys, nq, w.hist, order);
