@@ -43,7 +43,9 @@
 //     path index) -- word 0 the sample point, then one word per Russian
 //     roulette decision, as the reference draws them -- so results do not
 //     depend on launch shape, batching or query order.
-//   * The deeper steps of a query's surviving paths are added in path order and
+//   * The deeper steps of a query's surviving paths are added as a balanced tree
+//     per round, the rounds in order (one lane adding 32 paths in order held the
+//     warp for 32 shared loads a round), and
 //     divided by samples_per_subdomain once; the estimate is the first-level
 //     sum plus that.
 // With identical random decisions the estimator takes exactly the reference

@@ -21,7 +21,9 @@
 //                    D = -(m + log s) / alpha and its gradient -(g / s) / alpha.
 //
 // Each policy provides: V (the value type), zero(), nan(), add, sub, scale by a
-// float, div by a float, warp shuffles of a value (shfl, shfl_up), point() and
+// float, div by a float, warp shuffles of a value (shfl, shfl_up),
+// segment_scan() (the inclusive sum over a lane's segment of the warp: `head` its
+// first lane, `later` the first lanes of the segments after it), point() and
 // node() (the value of one source record or
 // node aggregate at query q), and store() (writes the result and, when the
 // caller asks, the gradient as structure-of-arrays [dim][nq]).  For sums whose
@@ -54,6 +56,15 @@ struct SumF {
   }
   __device__ __forceinline__ static V shfl_up(V a, int d) {
     return __shfl_up_sync(0xffffffffu, a, d);
+  }
+  __device__ __forceinline__ static V segment_scan(V x, int head, unsigned) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const V y = shfl_up(x, d);
+      if (lane - d >= head) x = add(y, x);
+    }
+    return x;
   }
   __device__ __forceinline__ static V point(float4 pm, float4 nr, float3 q, const KParams& kp) {
     return kernel_exact<DIM, K>(pm, nr, q, kp);
@@ -112,6 +123,15 @@ struct SumGrad {
     const unsigned f = 0xffffffffu;
     return V{__shfl_up_sync(f, a.v, d), __shfl_up_sync(f, a.gx, d), __shfl_up_sync(f, a.gy, d),
              DIM == 3 ? __shfl_up_sync(f, a.gz, d) : 0.f};
+  }
+  __device__ __forceinline__ static V segment_scan(V x, int head, unsigned) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const V y = shfl_up(x, d);
+      if (lane - d >= head) x = add(y, x);
+    }
+    return x;
   }
   __device__ __forceinline__ static V point(float4 pm, float4 nr, float3 q, const KParams& kp) {
     const float v = kernel_exact<DIM, K>(pm, nr, q, kp);
@@ -192,6 +212,32 @@ struct SumLse {
     const unsigned f = 0xffffffffu;
     return V{__shfl_up_sync(f, a.m, d), __shfl_up_sync(f, a.s, d), __shfl_up_sync(f, a.gx, d),
              __shfl_up_sync(f, a.gy, d), DIM == 3 ? __shfl_up_sync(f, a.gz, d) : 0.f};
+  }
+  // The terms of a segment are brought to its largest exponent first: one
+  // exponential a lane instead of one at each of the five steps of the scan.
+  __device__ __forceinline__ static V segment_scan(V x, int head, unsigned later) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    float top = x.m;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float y = __shfl_up_sync(full, top, d);
+      if (lane - d >= head) top = fmaxf(top, y);
+    }
+    top = __shfl_sync(full, top, later ? __ffs(later) - 2 : 31);
+    const float f = top == -__int_as_float(0x7f800000) ? 0.f : expf(x.m - top);
+    x = V{top, f * x.s, f * x.gx, f * x.gy, f * x.gz};
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const V y = shfl_up(x, d);
+      if (lane - d >= head) {
+        x.s += y.s;
+        x.gx += y.gx;
+        x.gy += y.gy;
+        if (DIM == 3) x.gz += y.gz;
+      }
+    }
+    return x;
   }
   __device__ __forceinline__ static V point(float4 pm, float4, float3 q, const KParams& kp) {
     const float dx = rsub(pm.x, q.x), dy = rsub(pm.y, q.y), dz = DIM == 3 ? rsub(pm.z, q.z) : 0.f;

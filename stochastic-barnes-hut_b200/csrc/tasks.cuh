@@ -437,13 +437,8 @@ __device__ __forceinline__ typename A::V expand(const DevTree& t, bool own, int 
       }
     }
     const bool counted = __any_sync(full, e < total && cnt != 1);
-    V x = val;
+    const V x = A::segment_scan(val, head, starts & ~upto);
     int cx = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const V y = A::shfl_up(x, d);
-      if (lane - d >= head) x = A::add(y, x);
-    }
     if (counted) {
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -558,16 +553,14 @@ struct SbhWarpSmem {
   // deeper path steps
   __device__ __forceinline__ int* qflag() const { return reinterpret_cast<int*>(base + 1056); }
   __device__ __forceinline__ int* qcount() const { return reinterpret_cast<int*>(base + 1088); }
-  // [32] a round's per-path sums, [32] per-query sums of the deeper steps and
-  // [32] per-query first-level sums
-  __device__ __forceinline__ V* pathv() const { return reinterpret_cast<V*>(base + 1120); }
-  __device__ __forceinline__ V* qsum() const { return reinterpret_cast<V*>(base + 1120 + 32 * W); }
-  __device__ __forceinline__ V* qacc() const { return reinterpret_cast<V*>(base + 1120 + 64 * W); }
+  // [32] per-query sums of the deeper steps and [32] per-query first-level sums
+  __device__ __forceinline__ V* qsum() const { return reinterpret_cast<V*>(base + 1120); }
+  __device__ __forceinline__ V* qacc() const { return reinterpret_cast<V*>(base + 1120 + 32 * W); }
 };
 
 template <class V>
 __host__ __device__ constexpr int sbh_warp_words() {
-  return 1120 + 96 * (int)(sizeof(V) / 4);
+  return 1120 + 64 * (int)(sizeof(V) / 4);
 }
 
 template <class V>
@@ -721,13 +714,13 @@ __device__ __forceinline__ long long sum_records_few(const DevTree& t, long long
 // k(c1), weighted) and the steps after it, exactly as in the reference loop
 // (include/tree_sampler.h:66-110).  Every lane decides its Russian roulette
 // step and finds its next node, then the warp expands all nodes the step needs
-// together (expand()).  Each path's sum of its steps is left in pathv[l]; the
-// contribution count of the round is returned on every lane.
+// together (expand()).  The paths' sum goes to round_sum and the contribution
+// count of the round is returned, both on every lane.
 template <int DIM, int K, class A>
 __device__ __forceinline__ int sbh_round(const DevTree& t, float3 q, long long key, int samples,
                                          unsigned long long seed, const KParams& kp,
                                          const SbhWarpSmem<typename A::V>& ws, int n, int* status,
-                                         bool& poisoned) {
+                                         bool& poisoned, typename A::V& round_sum) {
   using V = typename A::V;
   const int lane = threadIdx.x & 31;
   const int c0 = __ldg(t.nd_topo).x;
@@ -804,10 +797,9 @@ __device__ __forceinline__ int sbh_round(const DevTree& t, float3 q, long long k
       }
     }
   }
-  ws.pathv()[lane] = term;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  return cnt;
+  // The paths' sums added as a balanced tree (lanes beyond n hold zero).
+  round_sum = A::shfl(A::segment_scan(term, 0, 0u), 31);
+  return __reduce_add_sync(0xffffffffu, cnt);
 }
 
 // The stochastic estimator (multiLevelPrefixControlVariateSample_stackless,
@@ -894,7 +886,7 @@ __device__ __forceinline__ void sbh_warp_task(
     const long long key = key_base + qik;
     bool poisoned = false;
     int queued = 0, cntB = 0;
-    if (lane == 0) ws.qsum()[k] = A::zero();  // the surviving paths' deeper steps, in path order
+    if (lane == 0) ws.qsum()[k] = A::zero();  // the surviving paths' deeper steps, round by round
     for (int pbase = 0; pbase < P; pbase += 32) {
       // Bulk step, lane per path: sample the point, take the first step (out
       // of S, always taken) and the Russian roulette at the node c1 it leads
@@ -972,13 +964,10 @@ __device__ __forceinline__ void sbh_warp_task(
       const bool last = pbase + 32 >= P;
       while (queued >= 32 || (last && queued > 0)) {
         const int n = min(queued, 32);
-        cntB += sbh_round<DIM, K, A>(t, qk, key, samples, seed, kp, ws, n, status, poisoned);
+        V rsum;
+        cntB += sbh_round<DIM, K, A>(t, qk, key, samples, seed, kp, ws, n, status, poisoned, rsum);
         __syncwarp();
-        if (lane == 0) {
-          V dsum = ws.qsum()[k];
-          for (int r = 0; r < n; r++) dsum = A::add(dsum, ws.pathv()[r]);
-          ws.qsum()[k] = dsum;
-        }
+        if (lane == 0) ws.qsum()[k] = A::add(ws.qsum()[k], rsum);
         // move the waiting entries to the front
         for (int w = lane; w < (queued - n) * SbhWarpSmem<V>::kEntry; w += 32)
           ws.queue()[w] = ws.queue()[n * SbhWarpSmem<V>::kEntry + w];
