@@ -31,22 +31,19 @@
 //     path's sample point, its first step to the node c1 below S that holds the
 //     point (its path code gives the cell at every level) and the Russian
 //     roulette at c1; the few paths that continue go into a shared-memory queue.
-//     Whenever 32 are queued (and once at the end), the warp advances them in
-//     lock step: every lane decides its Russian roulette step and finds the
+//     When the queue (96 entries) could overflow, and once at the end, the warp
+//     runs the waiting paths in lock step, a lane taking the next one when its
+//     path ends: every lane decides its Russian roulette step and finds the
 //     next node, then the warp expands all nodes the step needs together -- the
 //     children of all those nodes as one flat list, 32 entries at a time
 //     (consecutive children are consecutive records, so the loads coalesce),
 //     and a segmented scan across the lanes forms every node's children sum.
-//     So rounds start full, instead of 32 paths of which most stop after one
-//     step waiting on the longest.
 //   * Each path draws its own Philox4x32-10 stream keyed by (seed, query index,
 //     path index) -- word 0 the sample point, then one word per Russian
 //     roulette decision, as the reference draws them -- so results do not
 //     depend on launch shape, batching or query order.
-//   * The deeper steps of a query's surviving paths are added as a balanced tree
-//     per round, the rounds in order (one lane adding 32 paths in order held the
-//     warp for 32 shared loads a round), and
-//     divided by samples_per_subdomain once; the estimate is the first-level
+//   * The deeper steps of a query's surviving paths are added by their lanes, the
+//     lanes as a balanced tree, and divided by samples_per_subdomain once; the estimate is the first-level
 //     sum plus that.
 // With identical random decisions the estimator takes exactly the reference
 // CPU estimator's paths and terms (each term rounded as the reference rounds

@@ -524,7 +524,7 @@ template <class V>
 struct SbhWarpSmem {
   float* base;
   static constexpr int W = (int)(sizeof(V) / 4);
-  static constexpr int kQueue = 64;  // survivor queue capacity (31 waiting + 32 new)
+  static constexpr int kQueue = 96;  // survivor queue capacity (63 waiting + 32 new)
   static constexpr int kEntry = 8;   // words per queue entry
   // [32] lanes of the current expansion's owners, in order
   __device__ __forceinline__ int* ownlane() const { return reinterpret_cast<int*>(base); }
@@ -542,25 +542,25 @@ struct SbhWarpSmem {
   // [32][8] records staged for the first-level sum: (x, y, z, mass), (normal,
   // flag); flag < 0 marks a leaf whose points are summed instead
   __device__ __forceinline__ float4* tile() const { return reinterpret_cast<float4*>(base + 288); }
-  // a row of terms per query where the warp holds few (FewQueries; over the tile
-  // and the queue below, both unused meanwhile)
+  // a row of terms per query where the warp holds few (FewQueries)
   __device__ __forceinline__ V* terms() const { return reinterpret_cast<V*>(base + 288); }
+  // (the queue takes the tile's and the terms' place after the first level)
   // [kQueue][kEntry] surviving paths: path index, sampled point, node to
   // expand, next node, path probability, running ratio, next node's depth,
   // pending random word
-  __device__ __forceinline__ int* queue() const { return reinterpret_cast<int*>(base + 544); }
+  __device__ __forceinline__ int* queue() const { return reinterpret_cast<int*>(base + 288); }
   // [32] per-query flags (bit 0: NaN result) and contribution counts of the
   // deeper path steps
-  __device__ __forceinline__ int* qflag() const { return reinterpret_cast<int*>(base + 1056); }
-  __device__ __forceinline__ int* qcount() const { return reinterpret_cast<int*>(base + 1088); }
+  __device__ __forceinline__ int* qflag() const { return reinterpret_cast<int*>(base + 288 + kQueue * kEntry); }
+  __device__ __forceinline__ int* qcount() const { return qflag() + 32; }
   // [32] per-query sums of the deeper steps and [32] per-query first-level sums
-  __device__ __forceinline__ V* qsum() const { return reinterpret_cast<V*>(base + 1120); }
-  __device__ __forceinline__ V* qacc() const { return reinterpret_cast<V*>(base + 1120 + 32 * W); }
+  __device__ __forceinline__ V* qsum() const { return reinterpret_cast<V*>(qflag() + 64); }
+  __device__ __forceinline__ V* qacc() const { return qsum() + 32; }
 };
 
 template <class V>
 __host__ __device__ constexpr int sbh_warp_words() {
-  return 1120 + 64 * (int)(sizeof(V) / 4);
+  return 288 + SbhWarpSmem<V>::kQueue * SbhWarpSmem<V>::kEntry + 64 + 64 * (int)(sizeof(V) / 4);
 }
 
 template <class V>
@@ -707,8 +707,10 @@ __device__ __forceinline__ long long sum_records_few(const DevTree& t, long long
   return cnt;
 }
 
-// One lock-step round over n (<= 32) surviving paths of one query, taken
-// from the front of the queue: lane l continues path l.  A survivor has taken
+// Lock-step steps over n surviving paths of one query, the queue's: every lane
+// continues one path and takes the next one waiting when its path ends, so the
+// steps stay full until the queue is empty (rounds of 32 that each ran to their
+// longest path, 79.3 -> 76.0 ms for 4M queries).  A survivor has taken
 // its first step (out of its subdomain S) and passed its Russian roulette at
 // the next node c1; what is left is c1's step (the children sum of c1 minus
 // k(c1), weighted) and the steps after it, exactly as in the reference loop
@@ -724,37 +726,46 @@ __device__ __forceinline__ int sbh_round(const DevTree& t, float3 q, long long k
   using V = typename A::V;
   const int lane = threadIdx.x & 31;
   const int c0 = __ldg(t.nd_topo).x;
-  const int* e = ws.queue() + lane * SbhWarpSmem<V>::kEntry;
-  bool own = lane < n, active = false;
+  bool own = false, active = false;
   int pid = 0, prev = 0, cur = 0, dcur = 0;
   float ev = 1.f, cb = 1.f;
   int4 tprev = make_int4(0, 0, 0, 0), tcur = tprev;
   PathRng rng;
   rng.n = 3;
-  if (own) {
-    pid = e[0];
-    const int idx = e[1];
-    prev = e[2];
-    cur = e[3];
-    ev = __int_as_float(e[4]);
-    cb = __int_as_float(e[5]);
-    dcur = e[6];
-    ws.rngbuf()[96 + lane] = (uint32_t)e[7];
-    const unsigned long long code = __ldg(t.pt_code + idx);
-    ws.path_code()[lane] = (uint32_t)code;
-    ws.path_code()[32 + lane] = (uint32_t)(code >> 32);
-    ws.path_point()[lane] = idx;
-    const int4 tS = __ldg(t.nd_topo + c0 + pid / samples);
-    ws.path_spi()[lane] = (float)(unsigned)(tS.w - tS.z);
-    const int4 tp4 = __ldg(t.nd_topo + prev);
-    tprev = make_int4(tp4.x, tp4.y, 0, 0);
-    const int4 tc4 = __ldg(t.nd_topo + cur);
-    tcur = make_int4(tc4.x, tc4.y, 0, 0);
-    active = tcur.y != 0;
-  }
   V term = A::zero();
   int cnt = 0;
-  while (__any_sync(0xffffffffu, own)) {
+  for (int next = 0;;) {
+    // Lanes without a path take the next ones waiting.
+    const unsigned idle = __ballot_sync(0xffffffffu, !own);
+    if (next < n && idle != 0u) {
+      const int mine = next + __popc(idle & ((1u << lane) - 1u));
+      if (!own && mine < n) {
+        const int* e = ws.queue() + mine * SbhWarpSmem<V>::kEntry;
+        own = true;
+        rng.n = 3;
+        pid = e[0];
+        const int idx = e[1];
+        prev = e[2];
+        cur = e[3];
+        ev = __int_as_float(e[4]);
+        cb = __int_as_float(e[5]);
+        dcur = e[6];
+        ws.rngbuf()[96 + lane] = (uint32_t)e[7];
+        const unsigned long long code = __ldg(t.pt_code + idx);
+        ws.path_code()[lane] = (uint32_t)code;
+        ws.path_code()[32 + lane] = (uint32_t)(code >> 32);
+        ws.path_point()[lane] = idx;
+        const int4 tS = __ldg(t.nd_topo + c0 + pid / samples);
+        ws.path_spi()[lane] = (float)(unsigned)(tS.w - tS.z);
+        const int4 tp4 = __ldg(t.nd_topo + prev);
+        tprev = make_int4(tp4.x, tp4.y, 0, 0);
+        const int4 tc4 = __ldg(t.nd_topo + cur);
+        tcur = make_int4(tc4.x, tc4.y, 0, 0);
+        active = tcur.y != 0;
+      }
+      next = min(n, next + __popc(idle));
+    }
+    if (!__any_sync(0xffffffffu, own)) break;
     // Paths of this round that stand at the same node need its children sum
     // once: the lowest such lane expands it and the others take its result.
     const unsigned same = __match_any_sync(0xffffffffu, own ? prev : -1 - lane);
@@ -959,18 +970,14 @@ __device__ __forceinline__ void sbh_warp_task(
       }
       queued += __popc(sm);
       __syncwarp();
-      // Full rounds while 32 or more paths wait; the rest wait for the next
-      // bulk step (or the final round).
+      // The waiting paths run when the next bulk step's might not fit, and at the end.
       const bool last = pbase + 32 >= P;
-      while (queued >= 32 || (last && queued > 0)) {
-        const int n = min(queued, 32);
+      if (queued > SbhWarpSmem<V>::kQueue - 32 || (last && queued > 0)) {
+        const int n = queued;
         V rsum;
         cntB += sbh_round<DIM, K, A>(t, qk, key, samples, seed, kp, ws, n, status, poisoned, rsum);
         __syncwarp();
         if (lane == 0) ws.qsum()[k] = A::add(ws.qsum()[k], rsum);
-        // move the waiting entries to the front
-        for (int w = lane; w < (queued - n) * SbhWarpSmem<V>::kEntry; w += 32)
-          ws.queue()[w] = ws.queue()[n * SbhWarpSmem<V>::kEntry + w];
         queued -= n;
         __syncwarp();
       }
