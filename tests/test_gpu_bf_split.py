@@ -30,3 +30,21 @@ def test_split_sums_match_fp64(n, nq, dim, kernel):
     ref = O.brute_force_f64(pts, nrm, m, kernel, q[nq - 1:], alpha=3.0)
     scale = O.brute_force_f64(pts, nrm, m, kernel, q[nq - 1:], alpha=3.0, abs_sum=True)
     assert abs(one[0] - ref[0]) <= 1e-6 * scale[0] and abs(v[-1] - ref[0]) <= 1e-6 * scale[0]
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_gravity_at_the_reciprocals_limits(dim):
+    """Distances beyond the shared reciprocal's range, at a source, infinite and NaN."""
+    rng = np.random.default_rng(6)
+    pts = rng.uniform(-1, 1, (515, dim)).astype(np.float32)
+    m = rng.uniform(-1, 1, 515).astype(np.float32)
+    lo, hi = W.padded_box(pts)
+    gpu = C.GpuTree(C.HostTree(pts, np.ones_like(pts), m, lo, hi))
+    q = np.array([[x] + [0.5] * (dim - 1) for x in
+                  (0.1, 9e8, 2e9, 1e15, 1.5e19, 3e19, 1e30, np.inf, np.nan)], np.float32)
+    q = np.concatenate([pts[7:8], q])
+    v, _ = gpu.eval(q, C.params(method=C.BRUTE_FORCE, kernel=C.GRAVITY))
+    scale = O.brute_force_f64(pts, np.ones_like(pts), m, C.GRAVITY, q[:6], abs_sum=True)
+    ref = O.brute_force_f64(pts, np.ones_like(pts), m, C.GRAVITY, q[:6])
+    assert (np.abs(v[:6] - ref) <= 1e-6 * scale).all()
+    assert (v[6:9] == 0).all() and np.isnan(v[9])  # r^2 overflows: terms of m / inf
