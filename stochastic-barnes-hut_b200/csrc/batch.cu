@@ -1,7 +1,8 @@
 // Batched evaluation: a list of requests -- each its own tree, method, kernel,
-// parameters and query count -- runs as one fixed pipeline, captured once as a
-// CUDA graph:
+// parameters and query count -- runs as one fixed pipeline, built once per launch
+// shape as a CUDA graph:
 //
+//   (the first four only where some request's queries are ordered)
 //   batch_bbox_kernel     the bounding box of every request's queries;
 //   batch_keys_kernel     Morton bucket of every query of every request, inside
 //                         its request's query box, with a per-request bucket
@@ -623,68 +624,84 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
   return "";
 }
 
-cudaError_t BatchEngine::capture(const DevTree* d_trees, int* d_status, const Shape& shape,
-                                 cudaGraphExec_t* out) {
+// Builds the pipeline's graph node by node.  (Capturing it from streams cost a
+// stream and an event per branch, 0.5 ms each, and any other thread's device
+// synchronisation -- a tree being destroyed -- invalidates a capture in progress.)
+cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
+                                     cudaGraphExec_t* out) {
   *out = nullptr;
-  // Captured on private streams (the caller's may be the legacy default
-  // stream, which cannot be captured); the graph is launched on the caller's.
-  // The query bucketing runs first, then the three class kernels as parallel
-  // branches of the graph: they share no state but the item table.
-  cudaStream_t st[1 + kClasses] = {};
-  cudaEvent_t ev[1 + kClasses] = {};
-  cudaError_t e = cudaSuccess;
-  for (int i = 0; i <= kClasses && e == cudaSuccess; i++) {
-    e = cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-  }
   cudaGraph_t graph = nullptr;
-  if (e == cudaSuccess) e = cudaStreamBeginCapture(st[0], cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    const int aux_blocks = sm_count_ * 4;
-    const int stack_cap = shape.bh_stack;
-    cudaMemsetAsync(d_hist_, 0, sizeof(unsigned) * max_buckets(lim_), st[0]);
-    cudaMemsetAsync(d_qbox_, 0, sizeof(unsigned) * 6 * lim_.max_items, st[0]);
-    batch_bbox_kernel<<<aux_blocks, kAuxThreads, 0, st[0]>>>(d_header_, d_items_, d_qbox_);
-    batch_keys_kernel<<<aux_blocks, kAuxThreads, 0, st[0]>>>(d_header_, d_items_, d_qbox_,
-                                                             d_keys_, d_hist_);
-    launch_scan(d_hist_, &d_header_->total_buckets, 0, max_buckets(lim_), d_sums_, st[0]);
-    batch_scatter_kernel<<<aux_blocks, kAuxThreads, 0, st[0]>>>(d_header_, d_items_, d_keys_,
-                                                                d_hist_, d_order_);
-    cudaEventRecord(ev[0], st[0]);
-    for (int c = 0; c < kClasses; c++) {
-      if (!((shape.classes >> c) & 1u)) continue;
-      cudaStream_t s = c == 0 ? st[0] : st[c];
-      if (c > 0) cudaStreamWaitEvent(s, ev[0], 0);
-      const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
-      const int fit = class_occupancy(c, smem);
-      const int per_sm = shape.per_sm_cap > 0 ? std::min(shape.per_sm_cap, fit) : fit;
-      const int blocks = per_sm * sm_count_;
-      const int words = class_warp_words(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
-      if (c == kClassBh)
-        batch_eval_kernel<kClassBh><<<blocks, kEvalThreads, smem, s>>>(
-            d_header_, d_items_, d_trees, d_order_, d_status, words, stack_cap);
-      else if (c == kClassSbh)
-        batch_eval_kernel<kClassSbh><<<blocks, kEvalThreads, smem, s>>>(
-            d_header_, d_items_, d_trees, d_order_, d_status, words, stack_cap);
-      else
-        kBfKernels[c - kClassBf]<<<blocks, kEvalThreads, smem, s>>>(
-            d_header_, d_items_, d_trees, words, d_partial_, d_counters_);
-      if (c > 0) {
-        cudaEventRecord(ev[c], s);
-        cudaStreamWaitEvent(st[0], ev[c], 0);
-      }
-    }
-    e = cudaStreamEndCapture(st[0], &graph);
+  cudaError_t e = cudaGraphCreate(&graph, 0);
+  if (e != cudaSuccess) return e;
+  using Nodes = std::vector<cudaGraphNode_t>;
+  auto clear = [&](void* p, size_t words) {
+    cudaGraphNode_t node = nullptr;
+    cudaMemsetParams m = {};
+    m.dst = p;
+    m.elementSize = 4;
+    m.width = words;
+    m.height = 1;
+    if (e == cudaSuccess) e = cudaGraphAddMemsetNode(&node, graph, nullptr, 0, &m);
+    return node;
+  };
+  // Arguments are copied into the node.
+  auto kernel = [&](const void* fn, unsigned grid, unsigned block, size_t smem, const Nodes& after,
+                    auto... args) {
+    cudaGraphNode_t node = nullptr;
+    void* ptrs[] = {&args...};
+    cudaKernelNodeParams k = {};
+    k.func = const_cast<void*>(fn);
+    k.gridDim = dim3(grid);
+    k.blockDim = dim3(block);
+    k.sharedMemBytes = (unsigned)smem;
+    k.kernelParams = ptrs;
+    if (e == cudaSuccess) e = cudaGraphAddKernelNode(&node, graph, after.data(), after.size(), &k);
+    return node;
+  };
+  auto fn = [](auto* f) { return reinterpret_cast<const void*>(f); };
+  const unsigned aux = sm_count_ * 4;
+  const BatchHeader* hdr = d_header_;
+  const BatchItem* items = d_items_;
+  const unsigned *qbox = d_qbox_, *keys = d_keys_;
+  Nodes ordered;
+  if (shape.sorted) {
+    const cudaGraphNode_t hist0 = clear(d_hist_, max_buckets(lim_));
+    const cudaGraphNode_t box0 = clear(d_qbox_, 6 * (size_t)lim_.max_items);
+    cudaGraphNode_t n =
+        kernel(fn(batch_bbox_kernel), aux, kAuxThreads, 0, {box0}, hdr, items, d_qbox_);
+    n = kernel(fn(batch_keys_kernel), aux, kAuxThreads, 0, {n, hist0}, hdr, items, qbox, d_keys_,
+               d_hist_);
+    // the scan of the buckets (launch_scan's three kernels)
+    const long long* buckets = &d_header_->total_buckets;
+    const long long fixed = 0;
+    const unsigned tiles = (unsigned)scan_tiles_for(max_buckets(lim_));
+    const unsigned *hist = d_hist_, *sums = d_sums_;
+    n = kernel(fn(scan_tile_sums), tiles, kScanThreads, 0, {n}, hist, buckets, fixed, d_sums_);
+    n = kernel(fn(scan_tile_offsets), 1, kScanThreads, 0, {n}, d_sums_, buckets, fixed);
+    n = kernel(fn(scan_tiles), tiles, kScanThreads, 0, {n}, d_hist_, buckets, fixed, sums);
+    n = kernel(fn(batch_scatter_kernel), aux, kAuxThreads, 0, {n}, hdr, items, keys, d_hist_,
+               d_order_);
+    ordered.push_back(n);
   }
-  for (int i = 0; i <= kClasses; i++) {
-    if (ev[i]) cudaEventDestroy(ev[i]);
-    if (st[i]) cudaStreamDestroy(st[i]);
+  // The classes' kernels, parallel branches: they share no state but the item
+  // table.  Only Barnes-Hut reads the ordering, but all start after it, Barnes-Hut
+  // first: its walks end one by one and brute force fills in behind them (the
+  // other way round the batch ends on the walks).
+  for (int c = 0; c < kClasses; c++) {
+    if (!((shape.classes >> c) & 1u)) continue;
+    const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
+    const int fit = class_occupancy(c, smem);
+    const unsigned blocks =
+        (unsigned)((shape.per_sm_cap > 0 ? std::min(shape.per_sm_cap, fit) : fit) * sm_count_);
+    const int words = class_warp_words(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
+    if (c < kClassBf)
+      kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items, d_trees,
+             (const int*)d_order_, d_status, words, shape.bh_stack);
+    else
+      kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items, d_trees, words,
+             d_partial_, d_counters_);
   }
-  if (e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    return e;
-  }
-  e = cudaGraphInstantiate(out, graph, 0);
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) *out = nullptr;
   return e;
@@ -712,6 +729,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   shape.sbh_root = round_root(need_root, lim_);
   for (const BatchItem& it : items) {
     shape.bh_query = shape.bh_query || it.per_query;
+    shape.sorted = shape.sorted || it.sort_bits > 0;
     shape.classes |= 1u << batch_class(it.method, it.dim, it.kernel);
   }
   cudaGraphExec_t exec = nullptr;
@@ -723,7 +741,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
         if (g.exec) cudaGraphExecDestroy(g.exec);
       graphs_.clear();
     }
-    cudaError_t e = capture(d_trees, d_status, shape, &exec);
+    cudaError_t e = build_graph(d_trees, d_status, shape, &exec);
     if (e != cudaSuccess) return e;
     graphs_.push_back(Graph{shape, exec});
   }

@@ -1,5 +1,5 @@
 // Batched evaluation: many requests (trees, kernels, methods, query counts) in
-// one persistent launch, captured as a CUDA graph.
+// one pipeline of persistent kernels, a CUDA graph.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -109,7 +109,7 @@ class BatchEngine {
                    const Tuning& tuning) const;
   // Enqueues the batch on `stream` (items already planned with `tuning`):
   // copies the item table and header from pinned staging, then launches the
-  // graph captured for the tuning's grid.
+  // graph of the batch's launch shape.
   cudaError_t launch(const std::vector<BatchItem>& items, const DevTree* d_trees,
                      int* d_status, cudaStream_t stream, const Tuning& tuning);
 
@@ -122,24 +122,25 @@ class BatchEngine {
   }
 
  private:
-  // What a captured pipeline is specialised for.
+  // What a pipeline's graph is specialised for.
   struct Shape {
     int per_sm_cap = 0;  // the tuning's CTAs-per-SM cap (0: none)
     int bh_stack = 0;    // Barnes-Hut stack entries per warp
     bool bh_query = false;  // whether the scratch holds bh_query_task's
     int sbh_root = 0;    // widest sampler root the scratch holds
     unsigned classes = 0;  // bit c: the batch has requests of class c
+    bool sorted = false;  // whether some request's queries are ordered
     bool operator==(const Shape& o) const {
       return per_sm_cap == o.per_sm_cap && bh_stack == o.bh_stack && bh_query == o.bh_query &&
-             sbh_root == o.sbh_root && classes == o.classes;
+             sbh_root == o.sbh_root && classes == o.classes && sorted == o.sorted;
     }
   };
   struct Graph {
     Shape shape;
     cudaGraphExec_t exec = nullptr;
   };
-  cudaError_t capture(const DevTree* d_trees, int* d_status, const Shape& shape,
-                      cudaGraphExec_t* out);
+  cudaError_t build_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
+                          cudaGraphExec_t* out);
 
   Limits lim_;
   int sm_count_;
@@ -158,7 +159,7 @@ class BatchEngine {
   unsigned* d_counters_ = nullptr;  // ... and how many of a tile's parts are done
   // pinned staging of header + items
   void* h_stage_ = nullptr;
-  // captured pipelines, one per launch shape
+  // instantiated pipelines, one per launch shape
   std::vector<Graph> graphs_;
   const DevTree* captured_trees_ = nullptr;
   int* captured_status_ = nullptr;

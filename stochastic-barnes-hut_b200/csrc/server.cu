@@ -1,7 +1,7 @@
 // C ABI: batched evaluation (sbh_eval_batch) and the serving loop (sbh_server_*).
 //
-// Both sit on BatchEngine (batch.cu): a fixed four-kernel pipeline captured
-// once as a CUDA graph, fed by one host-to-device copy of the request table.
+// Both sit on BatchEngine (batch.cu): a fixed pipeline built
+// once per launch shape as a CUDA graph, fed by one host-to-device copy of the request table.
 //
 // The server keeps trees resident and runs continuous batching over `slots`
 // batch contexts, each with its own stream, graph, device buffers sized to the
