@@ -53,8 +53,11 @@ __global__ void __launch_bounds__(BH_THREADS)
                                                   nullptr, stage);
 }
 
-// A warp per query (bh_query_task).  What bounds it is a step's chain of load,
-// test and compaction; 46-48 registers give 40 warps per SM to hide it.
+// A warp per query (bh_query_task).  Issue active 79% while an SM has work (65,536
+// queries, leaf 8), so what bounds it is the step's instructions; a third of the
+// time is the last walks' tail.  43-48 registers give 40 warps per SM.  Nodes and
+// leaf points of a step share one evaluation (two took 541 us instead of 456);
+// CTAs of 64 threads measured the same.
 template <int DIM, int K>
 __global__ void __launch_bounds__(BH_THREADS)
     barnes_hut_query_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,

@@ -14,9 +14,11 @@ cudaError_t launch_brute_force(const DevTree& t, int kernel, const float* q, lon
 // (bh_query_task), larger ones a lane per query (bh_warp_task).  A lane per query
 // does a node test in fewer instructions, but a call lasts at least as long as
 // its longest walk, one node after the other.  Measured on B200 (us, lane / warp
-// per query, theta 0.5): 1M-point torus, branching 64: 1,000 queries 3,482 / 205,
-// 65,536 5,054 / 1,015, 200,000 6,179 / 2,741, 1M 10,269 / 13,348; 10,000-point
-// Gaussian mixture, branching 8: 648 / 80, 810 / 227, 894 / 549, 1,315 / 2,550.
+// per query, theta 0.5): 1M-point torus, branching 64: 1,000 queries 2,910 / 170,
+// 65,536 4,206 / 1,032, 200,000 5,207 / 2,833, 300,000 5,252 / 4,194, 500,000 6,085 /
+// 6,950; 10,000-point Gaussian mixture, branching 8: 490 / 54, 603 / 236, 725 / 545,
+// 689 / 799, 751 / 1,290; 65,536 points, leaf 8: 1,414 / 282, 2,009 / 576, 2,298 /
+// 1,164, 2,370 / 1,635, 2,299 / 2,603.
 inline bool bh_query_per_warp(long long nq, int sm_count) { return nq <= 2048LL * sm_count; }
 // Without neighbours sharing a warp the query order only helps the L1 cache; up
 // to this many queries that is worth less than the ordering's seven launches

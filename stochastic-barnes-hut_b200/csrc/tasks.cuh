@@ -266,37 +266,34 @@ __device__ __forceinline__ void bh_query_task(const DevTree& t, const float* __r
     const int owner = owner_of[item ? head : 0] & 31;
     const int ea = __shfl_sync(full, e.a, owner), eb = __shfl_sync(full, e.b, owner);
     const int idx = ea + lane - head;
-    bool is_term = false, is_range = false;
+    bool eval = false, is_range = false;
     float val = 0.f;
     BhEntry r = BhEntry{0, 0};
-    if (item) {
-      if (eb > 0) {
-        const int4 topo = __ldg(t.nd_topo + idx);
-        const float4 cm = __ldg(t.nd_cm + idx);
-        const float4 ag = __ldg(t.nd_agg + idx);
-        const bool leaf = topo.y == 0;
-        const bool acc = leaf ? __int_as_float(0x7f800000) >= beta : far_enough<DIM>(cm, q, beta);
-        if (!acc) {
-          is_range = !leaf;
-          r = BhEntry{topo.x, topo.y};
-        } else if (leaf && topo.w - topo.z != 1) {
-          is_range = topo.w > topo.z;
-          r = BhEntry{topo.z, topo.z - topo.w};
-        } else {
-          const V v = A::node(cm, ag, q, kp);
-          is_term = A::kOrdered;
-          val = A::ordered(v);
-          rest = A::add_rest(rest, v);
-          nc++;
-        }
-      } else {
-        const V v = A::point(__ldg(t.pt_pm + idx), __ldg(t.pt_nrm + idx), q, kp);
-        is_term = A::kOrdered;
-        val = A::ordered(v);
-        rest = A::add_rest(rest, v);
-        nc++;
-      }
+    float4 src = make_float4(0.f, 0.f, 0.f, 0.f), nrm = src;  // the term's source, if it has one
+    if (item && eb > 0) {
+      const int4 topo = __ldg(t.nd_topo + idx);
+      const float4 cm = __ldg(t.nd_cm + idx);
+      const float4 ag = __ldg(t.nd_agg + idx);
+      const bool leaf = topo.y == 0;
+      const bool acc = leaf ? __int_as_float(0x7f800000) >= beta : far_enough<DIM>(cm, q, beta);
+      const bool points = leaf && topo.w - topo.z != 1;
+      eval = acc && !points;
+      is_range = acc ? points && topo.w > topo.z : !leaf;
+      r = acc ? BhEntry{topo.z, topo.z - topo.w} : BhEntry{topo.x, topo.y};
+      src = make_float4(cm.x, cm.y, cm.z, ag.x);
+      nrm = make_float4(ag.y, ag.z, ag.w, 0.f);
+    } else if (item) {
+      src = __ldg(t.pt_pm + idx);
+      nrm = __ldg(t.pt_nrm + idx);
+      eval = true;
     }
+    if (eval) {
+      const V v = A::point(src, nrm, q, kp);
+      val = A::ordered(v);
+      rest = A::add_rest(rest, v);
+      nc++;
+    }
+    const bool is_term = eval && A::kOrdered;
     // The window's outcomes in depth-first order: position of a node lane's own,
     // and of a waiting term's.
     const unsigned outs = __ballot_sync(full, is_term || is_range);
