@@ -18,13 +18,13 @@
 //   * aggregates are summed per node over its children in cell order (leaves:
 //     its single point), as tree3d.h:310-327 does.
 // What a build costs: 1,048,576 torus points, branching 64, take 4.0 ms, of which
-// the pageable host-to-device copy of 28 MB is 1.5, the kernels 1.1 and the tree's own
-// cudaMalloc 0.4.
+// the pageable host-to-device copy of 28 MB is 1.5 and the kernels 1.1.
 // The driver's calls were most of the 42 ms it took before -- about fifty
 // cudaMalloc/cudaFree pairs at 0.65 ms, a device property query at 2.5, a stream at
-// 0.5 -- so all scratch is one allocation from the library's pool.  On the device,
-// per-node histograms of all cells (217 MB at the widest level) became cell masks
-// and per-child counts, and levels of few nodes count in shared memory first.
+// 0.5 -- so the scratch and the tree are two allocations from the library's pool.
+// On the device, per-node histograms of all cells (217 MB at the widest level)
+// became cell masks and per-child counts, and levels of few nodes count in shared
+// memory first.
 //
 // For a leaf size above 1, or when the depth cap leaves several points in one
 // leaf, the order of the points inside a leaf is std::partition's and this
@@ -450,9 +450,6 @@ struct StreamCache {
 };
 StreamCache g_streams;
 
-// What the pool may keep of the builds' workspaces: a build of 4M points' worth.
-constexpr size_t kKeepBytes = size_t(1) << 30;
-
 // Builds on the device with room for `cap` nodes; SBH_ERR_UNSUPPORTED (nothing
 // kept) when the build needs the host (see the file comment), kMoreNodes when
 // cap was too small.
@@ -524,7 +521,7 @@ int build_with(Workspace& w, cudaStream_t s, size_t cap, int dsl, int leaf_size,
   g->device = device;
   g->sm_count = sm_count;
   g->bytes = L.bytes;
-  if (!ck(cudaMalloc(&g->mem, L.bytes))) what = "cudaMalloc(tree)";
+  if (!ck(sbh::alloc_tree_memory(device, L.bytes, s, &g->mem))) what = "tree memory";
   if (e == cudaSuccess) {
     sbh::bind_tree(g, L);
     char* base = static_cast<char*>(g->mem);
@@ -583,7 +580,8 @@ int build_with(Workspace& w, cudaStream_t s, size_t cap, int dsl, int leaf_size,
   if (e != cudaSuccess) {
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
-    cudaFree(g->mem);
+    cudaStreamSynchronize(s);
+    sbh::free_tree_memory(device, g->mem);
     delete g;
     return sbh::cuda_fail(e, what);
   }
@@ -619,7 +617,7 @@ int build_on_device(int dsl, int leaf_size, int max_depth, const float* points,
     cudaFreeAsync(mem, s);
     // nothing of a failed build may still read the caller's arrays
     cudaStreamSynchronize(s);
-    cudaMemPoolTrimTo(pool, kKeepBytes);
+    cudaMemPoolTrimTo(pool, sbh::kPoolKeepBytes);
     cap = std::min<size_t>(cap * 4, (size_t)INT32_MAX);
   } while (st == kMoreNodes);
   g_streams.give(device, s);

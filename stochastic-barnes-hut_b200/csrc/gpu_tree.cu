@@ -228,6 +228,21 @@ int sbh::scratch_pool(int device, cudaMemPool_t* out) {
   return SBH_OK;
 }
 
+cudaError_t sbh::alloc_tree_memory(int device, size_t bytes, cudaStream_t stream, void** out) {
+  *out = nullptr;
+  cudaMemPool_t pool = nullptr;
+  if (scratch_pool(device, &pool) != SBH_OK) return cudaErrorMemoryAllocation;
+  return cudaMallocFromPoolAsync(out, bytes, pool, stream);
+}
+
+void sbh::free_tree_memory(int device, void* mem) {
+  if (!mem) return;
+  cudaFreeAsync(mem, nullptr);
+  cudaStreamSynchronize(nullptr);
+  cudaMemPool_t pool = nullptr;
+  if (scratch_pool(device, &pool) == SBH_OK) cudaMemPoolTrimTo(pool, kPoolKeepBytes);
+}
+
 int sbh::check_device(int device, int* sm_count) {
   int major = 0, minor = 0;
   cudaError_t e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
@@ -302,10 +317,10 @@ SBH_API int sbh_gpu_tree_create(const sbh_host_tree* host, int device, sbh_gpu_t
   g->device = device;
   g->sm_count = sm_count;
   g->bytes = L.bytes;
-  cudaError_t e = cudaMalloc(&g->mem, L.bytes);
+  cudaError_t e = sbh::alloc_tree_memory(device, L.bytes, nullptr, &g->mem);
   if (e != cudaSuccess) {
     delete g;
-    return cuda_fail(e, "cudaMalloc(tree)");
+    return cuda_fail(e, "tree memory");
   }
   char* base = static_cast<char*>(g->mem);
   struct Copy {
@@ -328,7 +343,7 @@ SBH_API int sbh_gpu_tree_create(const sbh_host_tree* host, int device, sbh_gpu_t
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev1);
   if (e != cudaSuccess) {
     if (g->ev0) cudaEventDestroy(g->ev0);
-    cudaFree(g->mem);
+    sbh::free_tree_memory(device, g->mem);
     delete g;
     return cuda_fail(e, "tree upload");
   }
@@ -386,18 +401,19 @@ int sbh::clone_gpu_tree(const sbh_gpu_tree* src, sbh_gpu_tree** out) {
     g->box_lo[k] = src->box_lo[k];
     g->box_hi[k] = src->box_hi[k];
   }
-  cudaError_t e = cudaMalloc(&g->mem, src->bytes);
+  cudaError_t e = sbh::alloc_tree_memory(g->device, src->bytes, nullptr, &g->mem);
   if (e == cudaSuccess) e = cudaMemcpy(g->mem, src->mem, src->bytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev1);
   if (e != cudaSuccess) {
     if (g->ev0) cudaEventDestroy(g->ev0);
-    cudaFree(g->mem);
+    sbh::free_tree_memory(g->device, g->mem);
     delete g;
     return cuda_fail(e, "tree copy");
   }
   sbh::bind_tree(g, sbh::tree_layout(src->dev.n, src->dev.nn, src->dev.mw));
   cudaMemset(g->d_status, 0, sizeof(int));
+  cudaStreamSynchronize(nullptr);  // a copy within the device does not wait by itself
   *out = g;
   return SBH_OK;
 }
@@ -407,7 +423,7 @@ SBH_API void sbh_gpu_tree_destroy(sbh_gpu_tree* tree) {
   {
     DeviceGuard guard(tree->device);
     cudaDeviceSynchronize();
-    if (tree->mem) cudaFree(tree->mem);
+    sbh::free_tree_memory(tree->device, tree->mem);
     if (tree->ev0) cudaEventDestroy(tree->ev0);
     if (tree->ev1) cudaEventDestroy(tree->ev1);
   }
