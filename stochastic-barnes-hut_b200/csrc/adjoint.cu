@@ -63,8 +63,12 @@ __global__ void __launch_bounds__(AD_THREADS)
 
 // --------------------------------------------------------------- sampler ---
 
+// Seven CTAs per SM, with a few spills, hide more of the path steps' loads than the
+// five that the unbounded 96 registers allow (1M queries, 128 paths, us: 3D gravity
+// 17,567 -> 14,949, smooth distance 18,966 -> 17,301, Plummer 17,838 -> 14,719; 2D
+// 9,179 -> 8,925, 9,644 -> 9,709, 8,648 -> 8,625; eight: 2D Plummer 8,958).
 template <int DIM, int K, class A, bool FEW>
-__global__ void __launch_bounds__(AD_THREADS)
+__global__ void __launch_bounds__(AD_THREADS, 7)
     sbh_grad_kernel(DevTree t, const float* __restrict__ qsoa, long long nq,
                     int samples, unsigned long long seed, KParams kp, float* __restrict__ out, float* __restrict__ grads,
                     int* __restrict__ contribs, int* status, int group) {
