@@ -67,11 +67,11 @@ L2_FLUSH_BYTES = 512 << 20
 # figures are listed with the kernel's profile.  Null in the bench line when
 # the query count or budget is overridden.
 DRAM_TRAFFIC = {
-    "sbh_wn": 5.8709e9 + 0.2320e9,
-    "served_smooth": 194.35e6 + 7.80e6,
-    "bh_wn": 307.58e6 + 31.53e6,
-    "plain_small_bf": 1.85e6,
-    "plain_small_bh": 3.36e6,
+    "sbh_wn": 1.8481e9 + 0.1061e9,
+    "served_smooth": 183.71e6 + 5.93e6,
+    "bh_wn": 324.15e6 + 38.05e6,
+    "plain_small_bf": 1.87e6,
+    "plain_small_bh": 3.39e6,
 }
 
 # What each single-configuration workload measures (the headline metric is the
@@ -439,7 +439,7 @@ def run_ours(args, wl):
         bound, mufu_per_pair, fp32_per_pair = pair_pipe_bound(rates, wl["kernel"])
         pairs = float(nq) * float(wl["n"])
         roofline = {
-            "bound": "sfu", "kernel": "brute_force_kernel",
+            "bound": "sfu", "kernel": "split_sum_kernel",
             "achieved": pairs / kmean_s, "peak": bound,
             "unit": "pairs/s", "frac": pairs / kmean_s / bound,
             "peak_source": "measured MUFU rsqrt rate (sbh_measure_pipe_rates): "
@@ -465,7 +465,8 @@ def run_ours(args, wl):
             definition = (f"{bpe} B per kernel evaluation (node or point record) + 16 B per "
                           "query (SURVEY 8(d) per-unit figure; the opening tests' 32 B reads are "
                           "not counted)")
-            kernel_name = "barnes_hut_kernel"
+            # a warp per query in calls of up to 2,048 queries per SM, a lane per query beyond
+            kernel_name = "barnes_hut_query_kernel" if nq <= 2048 * 148 else "barnes_hut_kernel"
         roofline = {
             "bound": "issue", "kernel": kernel_name,
             "achieved": alg / kmean_s / 1e9, "peak": peak, "unit": "GB/s",
@@ -481,7 +482,8 @@ def run_ours(args, wl):
                     "DRAM traffic is a small fraction of HBM bandwidth); achieved/frac are the "
                     "requested load bandwidth against the HBM roof, dram_frac the DRAM share",
         }
-    launches_per_step = {"stochastic": 6, "barnes_hut": 6, "brute_force": 1}[wl["method"]]
+    # Barnes-Hut: the query ordering's seven kernels and the walk
+    launches_per_step = {"stochastic": 1, "barnes_hut": 8, "brute_force": 1}[wl["method"]]
     clk = clocks.summary()
     out = {
         "metric": WORKLOAD_METRIC[wl["name"]],
@@ -1236,7 +1238,7 @@ def run_serving(args):
         # per batch step: the graph's 9 kernels (query boxes, keys, three scan
         # kernels, scatter, one persistent kernel per method class) plus 8 (sort
         # and sampler) per stochastic request sent to its own launch
-        "gpu_launches": args.steps * (9 + 8 * n_direct),
+        "gpu_launches": args.steps * (9 + n_direct),
     }
 
 
@@ -1262,7 +1264,7 @@ def serving_breakdown(C, W, torch, trees, reqs, stream, flush):
         rates = C.measure_pipe_rates(0)
         peak, mufu_per_pair, fp32_per_pair = pair_pipe_bound(rates, top)
         achieved = p["pairs"] / (p["ms"] / 1e3)
-        roof = {"bound": "sfu", "kernel": "batch_eval_kernel (brute-force class), " + top,
+        roof = {"bound": "sfu", "kernel": "batch_bf_kernel, " + top,
                 "achieved": achieved, "peak": peak, "unit": "pairs/s", "frac": achieved / peak,
                 "peak_source": "measured MUFU rsqrt rate (sbh_measure_pipe_rates) / "
                                f"{mufu_per_pair} MUFU ops per pair (3D operation counts; "
@@ -1416,7 +1418,7 @@ def run_served_smooth(args):
                                f"stream (alpha 100, {nq} queries, {pairs:.3e} pairs) as one "
                                "sbh_eval_batch, queries resident, L2 flushed between steps"},
         "queries_per_s": nq / (kms / 1e3),
-        "roofline": {"bound": "sfu", "kernel": "batch_eval_kernel (brute-force class)",
+        "roofline": {"bound": "sfu", "kernel": "batch_bf_kernel (3D and 2D)",
                      "achieved": achieved, "peak": peak, "unit": "pairs/s",
                      "frac": achieved / peak,
                      "peak_source": "pair_pipe_bound per request dimension: measured MUFU rate "
@@ -1424,7 +1426,7 @@ def run_served_smooth(args):
                                     f"{rates['sm_clock_mhz']:.0f} MHz, 1.75 MUFU ops per pair",
                      "traffic": None if args.requests else DRAM_TRAFFIC.get("served_smooth")},
         "clocks": clocks.summary(),
-        "gpu_launches": args.steps * 9,
+        "gpu_launches": args.steps * 2,
     }
 
 

@@ -185,10 +185,10 @@ int sbh_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* queries,
 /* ---- evaluation, device buffers (asynchronous) -------------------------------
  * Same computation with d_queries/d_results (and optional d_contribs) in device
  * memory of the tree's device; enqueued on `stream`, returns without waiting.
- * Temporary device memory (the query order of Barnes-Hut and the sampler, about
- * 8 bytes per query) is allocated stream-ordered on `stream` from a memory pool
- * the library keeps per device; the pool holds on to freed memory, so it keeps
- * the largest call's scratch reserved until the process exits.  Device-side
+ * Temporary device memory (the query order of larger Barnes-Hut calls, about 8
+ * bytes per query) is allocated stream-ordered on `stream` from a memory pool
+ * the library keeps per device; the pool holds on to freed memory (tree builds
+ * and destructions trim what is free to 1 GiB).  Device-side
  * limit violations are reported by the next blocking call on the same tree, or
  * by sbh_gpu_tree_check. */
 int sbh_eval_device(sbh_gpu_tree* tree, const sbh_params* params, const float* d_queries,
@@ -198,8 +198,8 @@ int sbh_eval_device(sbh_gpu_tree* tree, const sbh_params* params, const float* d
  * No counterpart in the reference, which makes one launch (and one pair of
  * host-device copies) per call.  Evaluates many requests -- any trees resident
  * on one device, any methods, kernels, parameters and query counts -- in one
- * fixed pipeline captured once as a CUDA graph: Morton bucketing of all
- * requests' queries together, then one persistent work-queue kernel.  Per
+ * fixed pipeline built once as a CUDA graph: Morton bucketing of the requests'
+ * queries together, then persistent work-queue kernels, one per kind of request.  Per
  * request the results equal sbh_eval_device's: Barnes-Hut bit for bit, the
  * sampler because its random streams are keyed by (seed, query index within the
  * request).  Enqueued on `stream`; the call first waits for the previous batch
@@ -221,12 +221,13 @@ int sbh_eval_batch(const sbh_batch_item* items, int n_items, void* stream);
  * sampler's streams are keyed by query index, Barnes-Hut is exact per query);
  * only the speed does. */
 typedef struct sbh_batch_tuning {
-  int32_t sampler_unit_queries; /* sampler queries per work unit, 1..64 (default 32: the
-                                   first-level sum evaluates a unit's queries a lane each) */
+  int32_t sampler_unit_queries; /* sampler queries per work unit at most, 1..64 (default 32;
+                                   batches of few queries use smaller units) */
   int32_t bucket_queries;       /* target queries per Morton bucket, 2..4096 (default 8) */
   int32_t blocks_per_sm;        /* persistent CTAs per SM; 0 = as many as fit (default) */
   int32_t bh_unit_queries;      /* Barnes-Hut queries per warp walk, 1..32 (default 32; the
-                                   warp-vote method always uses 32) */
+                                   warp-vote method always uses 32, and short requests and
+                                   small batches run a warp per query instead) */
   int32_t direct_queries;       /* sbh_eval_batch: stochastic requests of at least this many
                                    queries run as their own sampler launches, on side streams
                                    beside the batch graph (same results); 0 = never (default
@@ -319,8 +320,8 @@ void sbh_server_destroy(sbh_server* server);
  * under memory pressure at any moment), or code whose device memory belongs to
  * another allocator's budget, such as a framework's caching allocator.
  * Limits and rules:
- *   - calls that order their queries (Barnes-Hut and stochastic without
- *     SBH_FLAG_KEEP_ORDER) take at most SBH_STATIC_SCRATCH_MAX_QUERIES queries;
+ *   - calls whose order of evaluation is left to the library (Barnes-Hut and
+ *     stochastic without SBH_FLAG_KEEP_ORDER) take at most SBH_STATIC_SCRATCH_MAX_QUERIES queries;
  *     larger counts return SBH_ERR_INVALID_ARGUMENT (split the batch).  Brute
  *     force, warp-vote Barnes-Hut and SBH_FLAG_KEEP_ORDER calls use no scratch
  *     and take any count;
