@@ -602,11 +602,16 @@ int build_on_device(int dsl, int leaf_size, int max_depth, const float* points,
   if (st != SBH_OK) return st;
   cudaStream_t s = g_streams.take(device);
   if (!s) return sbh::cuda_fail(cudaGetLastError(), "cudaStreamCreate");
-  size_t cap = 2 * (size_t)n + 4096;
+  size_t cap = std::min<size_t>(2 * (size_t)n + 4096, (size_t)INT32_MAX);
   do {
     const size_t bytes = carve(nullptr, DIM, n, cap, mw).bytes;
     void* mem = nullptr;
     cudaError_t e = cudaMallocFromPoolAsync(&mem, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) {  // the host build needs the tree's memory alone
+      cudaGetLastError();
+      st = SBH_ERR_UNSUPPORTED;
+      break;
+    }
     if (e != cudaSuccess) {
       st = sbh::cuda_fail(e, "cudaMallocFromPoolAsync(tree build)");
       break;
