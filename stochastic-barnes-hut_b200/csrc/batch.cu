@@ -214,9 +214,8 @@ __device__ __noinline__ void run_bh_query(const DevTree& t, const BatchItem& it,
 // Brute force: a tile of kBfTileQueries queries against all parts of the sources
 // (bf_parts), or, of a split request, against one of them; one warp
 // (lane_sum.cuh).  The sums of one part go to `partials` ([tile][part][query]) and
-// the tile's last unit, by its counter, merges them in part order and stores; it
-// leaves the counter at zero.  `tot` is the warp's scratch of kBfTileQueries
-// sums.  The request's fields are read where they are needed, not carried
+// the tile's last unit, by its counter (at zero when the batch starts), merges them
+// in part order and stores.  `tot` is the warp's scratch of kBfTileQueries sums.  The request's fields are read where they are needed, not carried
 // through the sums' registers.
 template <int DIM, int K>
 __device__ __forceinline__ void run_bf(const DevTree& t, const BatchItem& it, long long u,
@@ -263,7 +262,6 @@ __device__ __forceinline__ void run_bf(const DevTree& t, const BatchItem& it, lo
     before = __shfl_sync(0xffffffffu, before, 0);
     if (before + 1 != (unsigned)it.split) return;
     __threadfence();
-    if (lane == 0) *counter = 0u;
     for (int p = 0; p < it.split; p++) {
       const float2 x = __ldcg(sums + p * kBfTileQueries + (lane & (kBfTileQueries - 1)));
       const PlainSum y = {x.x, x.y};
@@ -502,8 +500,6 @@ BatchEngine::BatchEngine(const Limits& lim, int sm_count) : lim_(lim), sm_count_
   d_sums_ = reinterpret_cast<unsigned*>(b + o_sums);
   d_partial_ = reinterpret_cast<PlainSum*>(b + o_partial);
   d_counters_ = reinterpret_cast<unsigned*>(b + o_counters);
-  // at zero between batches: a tile's last unit puts its counter back
-  cudaMemset(d_counters_, 0, sizeof(unsigned) * kMaxTileParts / 2);
   if (cudaMallocHost(&h_stage_, o_keys) != cudaSuccess) h_stage_ = nullptr;
   // Allow each class's kernel the shared memory of the engine's largest
   // shape; report occupancy at the smallest (the register bound).
@@ -746,6 +742,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
     graphs_.push_back(Graph{shape, exec});
   }
   BatchHeader h = {};
+  long long split_tiles = 0;
   h.n_items = (int)items.size();
   for (int c = 0; c < kClasses; c++) h.item_begin[c] = h.item_end[c] = 0;
   int prev = -1;
@@ -760,6 +757,7 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
     h.total_queries += it.nq;
     h.total_buckets += it.buckets;
     h.total_units[c] += it.units;
+    if (it.split) split_tiles += it.units / it.split;
   }
   char* st = static_cast<char*>(h_stage_);
   std::memcpy(st, &h, sizeof(h));
@@ -767,6 +765,11 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   if (!items.empty()) std::memcpy(st + o_items, items.data(), sizeof(BatchItem) * items.size());
   cudaError_t e = cudaMemcpyAsync(d_header_, st, o_items + sizeof(BatchItem) * items.size(),
                                   cudaMemcpyHostToDevice, stream);
+  // The counters of this batch's split tiles, on the stream that runs it: nothing
+  // else orders a clearing before a batch (the default stream's work does not come
+  // before a non-blocking stream's).
+  if (e == cudaSuccess && split_tiles > 0)
+    e = cudaMemsetAsync(d_counters_, 0, sizeof(unsigned) * split_tiles, stream);
   if (e != cudaSuccess) return e;
   return cudaGraphLaunch(exec, stream);
 }
