@@ -411,12 +411,15 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
     const int stack_cap = t.depth + 2;
     const size_t smem = (size_t)AD_WARPS * stack_cap * sizeof(BhStackEntry);
     const long long blocks = (nq + AD_THREADS - 1) / AD_THREADS;
-    if (method == SBH_METHOD_BARNES_HUT_VOTE)
-      bh_grad_kernel<DIM, K, true, A><<<(unsigned)blocks, AD_THREADS, smem, stream>>>(
-          t, q, nq, order, beta, kp, out, grads, contribs, status, stack_cap);
-    else
-      bh_grad_kernel<DIM, K, false, A><<<(unsigned)blocks, AD_THREADS, smem, stream>>>(
-          t, q, nq, order, beta, kp, out, grads, contribs, status, stack_cap);
+    const auto kernel = method == SBH_METHOD_BARNES_HUT_VOTE ? bh_grad_kernel<DIM, K, true, A>
+                                                             : bh_grad_kernel<DIM, K, false, A>;
+    if (smem > 48 * 1024) {  // trees deeper than 766
+      cudaError_t e =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    kernel<<<(unsigned)blocks, AD_THREADS, smem, stream>>>(t, q, nq, order, beta, kp, out, grads,
+                                                           contribs, status, stack_cap);
     return cudaGetLastError();
   }
   using V = typename A::V;
