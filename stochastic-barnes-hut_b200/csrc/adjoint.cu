@@ -119,9 +119,10 @@ struct CompSum<SumGrad<DIM, K>> {
 template <int DIM>
 struct CompSum<SumLse<DIM>> {
   LseValue hi = SumLse<DIM>::zero(), lo{0.f, 0.f, 0.f, 0.f, 0.f};
+  // A NaN exponent takes the first branch, here and at every later addition, and stays
+  // NaN in s; a zero (m = -inf) adds nothing without a branch of its own.
   __device__ __forceinline__ void add(LseValue p) {
-    if (p.m == -__int_as_float(0x7f800000)) return;
-    if (p.m > hi.m) {
+    if (!(p.m <= hi.m)) {
       const float f = hi.m == -__int_as_float(0x7f800000) ? 0.f : expf(hi.m - p.m);
       hi = LseValue{p.m, hi.s * f, hi.gx * f, hi.gy * f, hi.gz * f};
       lo = LseValue{p.m, lo.s * f, lo.gx * f, lo.gy * f, lo.gz * f};
@@ -135,7 +136,6 @@ struct CompSum<SumLse<DIM>> {
     two_sum_into(hi.gz, lo.gz, p.gz);
   }
   __device__ __forceinline__ void merge(const CompSum& b) {
-    if (b.hi.m == -__int_as_float(0x7f800000)) return;
     add(b.hi);
     const float f = b.hi.m == hi.m ? 1.f : expf(b.hi.m - hi.m);
     lo = LseValue{hi.m, lo.s + f * b.lo.s, lo.gx + f * b.lo.gx, lo.gy + f * b.lo.gy,

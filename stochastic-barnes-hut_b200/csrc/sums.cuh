@@ -166,6 +166,13 @@ struct LseValue {
   float m, s, gx, gy, gz;
 };
 
+// The larger of two, NaN if either is.
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
 // Smooth distance exp(-alpha r): exponent t = -alpha r, gradient of t
 // alpha (p - q) / r (0 at r = 0); a term is (t, 1, grad t).
 template <int DIM>
@@ -183,8 +190,9 @@ struct SumLse {
     const float n = __int_as_float(0x7fc00000);
     return V{n, n, n, n, n};
   }
+  // A NaN stays in m: a zero's m, -inf, would otherwise be taken for "nothing here".
   __device__ __forceinline__ static V add(V a, V b) {
-    if (a.m < b.m) {
+    if (a.m < b.m || b.m != b.m) {
       const V t = a;
       a = b;
       b = t;
@@ -222,10 +230,10 @@ struct SumLse {
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const float y = __shfl_up_sync(full, top, d);
-      if (lane - d >= head) top = fmaxf(top, y);
+      if (lane - d >= head) top = max_or_nan(top, y);
     }
     top = __shfl_sync(full, top, later ? __ffs(later) - 2 : 31);
-    const float f = top == -__int_as_float(0x7f800000) ? 0.f : expf(x.m - top);
+    const float f = x.m == -__int_as_float(0x7f800000) ? 0.f : expf(x.m - top);
     x = V{top, f * x.s, f * x.gx, f * x.gy, f * x.gz};
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -243,7 +251,7 @@ struct SumLse {
     const float dx = rsub(pm.x, q.x), dy = rsub(pm.y, q.y), dz = DIM == 3 ? rsub(pm.z, q.z) : 0.f;
     // The exponent exactly as the plain kernel forms it (include/kernel.h:55-58).
     const float r = rsqrt_ieee(dot_exact<DIM>(dx, dy, dz, dx, dy, dz));
-    const float c = r > 0.f ? kp.alpha / r : 0.f;
+    const float c = r == 0.f ? 0.f : kp.alpha / r;
     return V{rmul(-kp.alpha, r), 1.f, rmul(c, dx), rmul(c, dy), rmul(c, dz)};
   }
   __device__ __forceinline__ static V node(float4 cm, float4 agg, float3 q, const KParams& kp) {
