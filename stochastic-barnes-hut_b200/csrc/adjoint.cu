@@ -215,9 +215,11 @@ struct GradBase {
   QueryPairs<NP> q;
   Sum total[Q];
   KParams kp;
+  // The policy's addition drops a term e^-inf, whose gradient may be NaN (0 times an
+  // infinite distance); the compensated sum would keep it.
   __device__ __forceinline__ void single(float4 s, float4 n) {
 #pragma unroll
-    for (int j = 0; j < Q; j++) total[j].add(A::point(s, n, q.query(j), kp));
+    for (int j = 0; j < Q; j++) total[j].add(A::add(A::zero(), A::point(s, n, q.query(j), kp)));
   }
   __device__ __forceinline__ const Sum& sum(int j) const { return total[j]; }
   __device__ __forceinline__ static void store(float* out, float* grads, long long nq,
