@@ -151,8 +151,8 @@ struct CompSum<SumLse<DIM>> {
 // FP32 pipes together (two MUFU and about 16 FP32 operations a pair).  Two pairs
 // a warp; one measured 1.1 to 2.1 times the time.  Against a query per thread with
 // IEEE roots and divisions (us): 4,001 queries x 262,144 sources in 2D, smooth
-// distance 34,550 -> 897, gravity 47,130 -> 691, Plummer 42,081 -> 504; 30,000 x
-// 65,536 in 3D 10,818 -> 2,344, 12,826 -> 1,608, 11,269 -> 1,216.  A group of sources is
+// distance 34,550 -> 867, gravity 47,130 -> 691, Plummer 42,081 -> 504; 30,000 x
+// 65,536 in 3D 10,818 -> 2,207, 12,826 -> 1,608, 11,269 -> 1,216.  A group of sources is
 // summed on its own first: a term outside the fast form's range (a source at the
 // query, distances whose square leaves the FP32 normal range, NaN) makes the
 // group's sum infinite or NaN, and that query's group is then evaluated term by
@@ -299,8 +299,13 @@ struct GradAcc : GradBase<DIM, A, NP> {
 };
 
 // Smooth distance: terms e^(t - m), t = -alpha r, against a query's own reference
-// exponent m, raised when a group's largest t is 40 above it (so terms stay below
-// e^40, and what flushes to zero is below e^-47 of the largest term).
+// exponent m, raised when a group's largest t is kLag above it.  The MUFU's argument
+// (t - m) log2 e is rounded at its own magnitude, so what m may lag behind the terms
+// that count is a relative error of those terms.  Measured with the nearest sources 39
+// above the first ones (median gradient error against FP64, 3D; 4,001 queries x 262,144
+// sources in 2D, us): kLag 40 4.7e-7, 816; 8 6.7e-8, 839; 4 6.7e-8, 867; 2 6.7e-8,
+// 907; 0 6.7e-8, 975; a running maximum with IEEE operations 7.1e-8.  What flushes to
+// zero is below e^-83 of the largest term.
 template <int DIM, class A, int NP>
 struct GradAcc<DIM, kSmoothDist, A, NP> : GradBase<DIM, A, NP> {
   using GradBase<DIM, A, NP>::q;
@@ -317,9 +322,10 @@ struct GradAcc<DIM, kSmoothDist, A, NP> : GradBase<DIM, A, NP> {
       s_[p] = gx[p] = gy[p] = gz[p] = dup(0.f);
     }
   }
+  static constexpr float kLag = 4.f;
   // Factor that takes sums from reference exponent m to the higher one, tm.
   __device__ __forceinline__ static float raise(float& m, float tm) {
-    if (!(tm > m + 40.f) || !usable(tm)) return 1.f;
+    if (!(tm > m + kLag) || !usable(tm)) return 1.f;
     const float f = expf(m - tm);
     m = tm;
     return f;
@@ -340,7 +346,7 @@ struct GradAcc<DIM, kSmoothDist, A, NP> : GradBase<DIM, A, NP> {
       }
       const float tx = fmaxf(fmaxf(t[0].x, t[1].x), fmaxf(t[2].x, t[3].x));
       const float ty = fmaxf(fmaxf(t[0].y, t[1].y), fmaxf(t[2].y, t[3].y));
-      if (tx > m[p].x + 40.f || ty > m[p].y + 40.f) {
+      if (tx > m[p].x + kLag || ty > m[p].y + kLag) {
         const float2 f = make_float2(raise(m[p].x, tx), raise(m[p].y, ty));
         s_[p] = __fmul2_rn(s_[p], f);
         gx[p] = __fmul2_rn(gx[p], f);
@@ -382,6 +388,15 @@ struct GradAcc<DIM, kSmoothDist, A, NP> : GradBase<DIM, A, NP> {
       total[2 * p + 1].add(LseValue{m[p].y, s_[p].y, al * gx[p].y, al * gy[p].y, al * gz[p].y});
       s_[p] = gx[p] = gy[p] = gz[p] = dup(0.f);
     }
+  }
+  // The value's logarithm and its addition in FP64, one per query: m lies below the
+  // largest term, log s is larger for it, and its FP32 rounding showed (value errors up
+  // to 1.1 times a running maximum's, now 0.4 to 0.8).
+  __device__ __forceinline__ static void store(float* out, float* grads, long long nq,
+                                               long long qi, const CompSum<A>& s,
+                                               const KParams& kp) {
+    A::store(out, grads, nq, qi, s.result(), kp);
+    out[qi] = (float)(-(s.hi.m + log((double)s.hi.s + s.lo.s)) / kp.alpha);
   }
 };
 
