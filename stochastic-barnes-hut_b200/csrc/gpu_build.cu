@@ -622,7 +622,7 @@ int build_on_device(int dsl, int leaf_size, int max_depth, const float* points,
     cudaFreeAsync(mem, s);
     // nothing of a failed build may still read the caller's arrays
     cudaStreamSynchronize(s);
-    cudaMemPoolTrimTo(pool, sbh::kPoolKeepBytes);
+    sbh::trim_pool(pool);
     cap = std::min<size_t>(cap * 4, (size_t)INT32_MAX);
   } while (st == kMoreNodes);
   g_streams.give(device, s);

@@ -80,6 +80,11 @@ constexpr size_t kPoolKeepBytes = size_t(1) << 30;
 cudaError_t alloc_tree_memory(int device, size_t bytes, cudaStream_t stream, void** out);
 void free_tree_memory(int device, void* mem);
 
+// Returns what is free in the pool beyond kPoolKeepBytes to the driver.  (What
+// cudaMemPoolTrimTo keeps counts the memory in use: resident trees would use the
+// allowance up.)
+void trim_pool(cudaMemPool_t pool);
+
 // Whether `device` (a valid index) runs this build's code; its SM count.  Two
 // attribute reads: the whole property record takes the driver 2.5 ms.
 int check_device(int device, int* sm_count);

@@ -240,7 +240,13 @@ void sbh::free_tree_memory(int device, void* mem) {
   cudaFreeAsync(mem, nullptr);
   cudaStreamSynchronize(nullptr);
   cudaMemPool_t pool = nullptr;
-  if (scratch_pool(device, &pool) == SBH_OK) cudaMemPoolTrimTo(pool, kPoolKeepBytes);
+  if (scratch_pool(device, &pool) == SBH_OK) trim_pool(pool);
+}
+
+void sbh::trim_pool(cudaMemPool_t pool) {
+  uint64_t used = 0;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, used + kPoolKeepBytes);
 }
 
 int sbh::check_device(int device, int* sm_count) {
