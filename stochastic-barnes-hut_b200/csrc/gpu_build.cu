@@ -451,8 +451,8 @@ struct StreamCache {
 StreamCache g_streams;
 
 // Builds on the device with room for `cap` nodes; SBH_ERR_UNSUPPORTED (nothing
-// kept) when the build needs the host (see the file comment), kMoreNodes when
-// cap was too small.
+// kept) when the build needs the host (see the file comment) or the tree does not
+// fit beside the workspace, kMoreNodes when cap was too small.
 constexpr int kMoreNodes = -1;
 
 template <int DIM>
@@ -522,6 +522,11 @@ int build_with(Workspace& w, cudaStream_t s, size_t cap, int dsl, int leaf_size,
   g->sm_count = sm_count;
   g->bytes = L.bytes;
   if (!ck(sbh::alloc_tree_memory(device, L.bytes, s, &g->mem))) what = "tree memory";
+  if (e == cudaErrorMemoryAllocation) {  // it may fit without the workspace
+    cudaGetLastError();
+    delete g;
+    return SBH_ERR_UNSUPPORTED;
+  }
   if (e == cudaSuccess) {
     sbh::bind_tree(g, L);
     char* base = static_cast<char*>(g->mem);
