@@ -215,14 +215,22 @@ __device__ __forceinline__ int nth_cell(const Nodes& nd, int v, int k) {
   return w * 64 + b;
 }
 
+// The node of its level that a thread of k_children works on, eight lanes a node: a
+// level of 2^29 nodes has as many threads as 32 bits can number.
+__host__ __device__ constexpr long long child_thread_node(unsigned block, unsigned thread) {
+  return ((long long)block * kThreads + thread) / 8;
+}
+static_assert(child_thread_node(1u << 24, 8) == (1LL << 29) + 1, "thread numbers beyond 32 bits");
+
 // Child nodes of the level's split nodes (tree3d.h:291-301): ranges, bounds
 // min + i*inc (include/aabb.h).  Eight lanes per node, a child each at a time.
 template <int DIM>
 __global__ void k_children(Nodes nd, int lb, int le, int dsl) {
-  const int v = lb + (blockIdx.x * blockDim.x + threadIdx.x) / 8;
+  const long long at = lb + child_thread_node(blockIdx.x, threadIdx.x);
   const int l = threadIdx.x & 7;
-  const int nch = v < le ? nd.nch[v] : 0;
+  const int nch = at < le ? nd.nch[at] : 0;
   if (nch == 0) return;  // the same for the node's eight lanes
+  const int v = (int)at;
   const unsigned group = 0xffu << (threadIdx.x & 24);
   const int ds = 1 << dsl;
   const float4 lo = nd.bmin[v], hi = nd.bmax[v];
