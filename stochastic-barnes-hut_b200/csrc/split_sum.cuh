@@ -111,30 +111,36 @@ inline SplitShape split_shape(long long nq, long long n, int q_per_warp, int cta
   return best;
 }
 
+// A cluster of 16 is more than every context must be able to place (8 is not): where
+// one cannot, the launch is refused and the call runs in clusters of 8.
 template <class Acc, int DIM>
 cudaError_t launch_split(const DevTree& t, const float* q, long long nq, const KParams& kp,
                          float* out, float* grads, int* contribs, cudaStream_t stream,
                          const SplitShape& shape) {
   const long long per_cta = (long long)(kSplitWarps / shape.sw) * Acc::Q;
   const long long tiles = (nq + per_cta - 1) / per_cta;
-  if (shape.csize > 8) {
-    cudaError_t e = cudaFuncSetAttribute(split_sum_kernel<Acc, DIM>,
-                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * shape.csize), 1, 1);
-  cfg.blockDim = dim3(kSplitThreads, 1, 1);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = shape.csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, split_sum_kernel<Acc, DIM>, t, q, nq, kp, shape.sw, out, grads,
-                            contribs);
+  auto launch = [&](int csize) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * csize), 1, 1);
+    cfg.blockDim = dim3(kSplitThreads, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, split_sum_kernel<Acc, DIM>, t, q, nq, kp, shape.sw, out, grads,
+                              contribs);
+  };
+  if (shape.csize <= 8) return launch(shape.csize);
+  cudaError_t e = cudaFuncSetAttribute(split_sum_kernel<Acc, DIM>,
+                                       cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = launch(shape.csize);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  return launch(8);
 }
 
 }  // namespace
