@@ -399,20 +399,19 @@ __global__ void __launch_bounds__(kEvalThreads, 4)
 
 // Per-warp shared words of a class's kernel for a launch shape: the tree and
 // request records, then the class's scratch (Barnes-Hut stack of `bh_stack`
-// entries or bh_query_task's scratch, or sampler scratch for roots of up to `sbh_r` children).
-int class_warp_words(int cls, int bh_stack, bool bh_query, int sbh_r) {
+// entries or bh_query_task's scratch, or the sampler's).
+int class_warp_words(int cls, int bh_stack, bool bh_query) {
   int scratch = 0;
   if (cls == kClassBh) scratch = bh_stack * (int)sizeof(BhStackEntry) / 4;
   if (cls == kClassBh && bh_query)
     scratch = std::max(scratch, (int)(bh_query_smem(bh_stack) / 4));
   if (cls == kClassSbh) scratch = sbh_warp_words<float>();
   if (cls >= kClassBf) scratch = kBfTileQueries * (int)sizeof(PlainSum) / 4;
-  (void)sbh_r;
   return kTreeWords + kItemWords + (scratch + 3) / 4 * 4;
 }
 
-size_t class_smem(int cls, int bh_stack, bool bh_query, int sbh_r) {
-  return (size_t)kEvalWarps * class_warp_words(cls, bh_stack, bh_query, sbh_r) * sizeof(float);
+size_t class_smem(int cls, int bh_stack, bool bh_query) {
+  return (size_t)kEvalWarps * class_warp_words(cls, bh_stack, bh_query) * sizeof(float);
 }
 
 using BfKernel = void (*)(BatchHeader*, const BatchItem*, const DevTree*, int, PlainSum*, unsigned*);
@@ -440,16 +439,11 @@ int class_occupancy(int cls, size_t smem) {
 }
 
 // Launch shapes are rounded so that few graphs serve every batch: the stack
-// to a multiple of 32 entries, the root width to a power of two from 64.
+// to a multiple of 32 entries.
 // Shared memory sized to the batch (not to the engine's limits) leaves the
 // rest of each SM's 228 KB to the L1 cache the traversals depend on.
 int round_stack(int need, const BatchEngine::Limits& lim) {
   return std::min((need + 31) / 32 * 32, lim.max_tree_depth + 2);
-}
-int round_root(int need, const BatchEngine::Limits& lim) {
-  int r = 64;
-  while (r < need) r *= 2;
-  return std::min(r, lim.max_root_children);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -503,16 +497,14 @@ BatchEngine::BatchEngine(const Limits& lim, int sm_count) : lim_(lim), sm_count_
   if (cudaMallocHost(&h_stage_, o_keys) != cudaSuccess) h_stage_ = nullptr;
   // Allow each class's kernel the shared memory of the engine's largest
   // shape; report occupancy at the smallest (the register bound).
-  const int big_stack = lim_.max_tree_depth + 2, big_root = lim_.max_root_children;
-  for (int c = 0; c < kClasses; c++) allow_smem(c, class_smem(c, big_stack, true, big_root));
-  const int small_stack = round_stack(0, lim_), small_root = round_root(0, lim_);
+  const int big_stack = lim_.max_tree_depth + 2, small_stack = round_stack(0, lim_);
+  for (int c = 0; c < kClasses; c++) allow_smem(c, class_smem(c, big_stack, true));
   for (int c = 0; c < kClasses; c++)
-    per_sm_[c] = class_occupancy(c, class_smem(c, small_stack, false, small_root));
+    per_sm_[c] = class_occupancy(c, class_smem(c, small_stack, false));
 }
 
 BatchEngine::~BatchEngine() {
-  for (Graph& g : graphs_)
-    if (g.exec) cudaGraphExecDestroy(g.exec);
+  for (Graph& g : graphs_) release(g);
   if (h_stage_) cudaFreeHost(h_stage_);
   if (dev_) cudaFree(dev_);
 }
@@ -620,15 +612,22 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
   return "";
 }
 
-// Builds the pipeline's graph node by node.  (Capturing it from streams cost a
-// stream and an event per branch, 0.5 ms each, and any other thread's device
-// synchronisation -- a tree being destroyed -- invalidates a capture in progress.)
-cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
-                                     cudaGraphExec_t* out) {
-  *out = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaGraphCreate(&graph, 0);
+void BatchEngine::release(Graph& g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+  g.exec = nullptr;
+  g.graph = nullptr;
+}
+
+// Builds the pipeline's graph of g's shape and classes node by node.  (Capturing it
+// from streams cost a stream and an event per branch, 0.5 ms each, and any other
+// thread's device synchronisation -- a tree being destroyed -- invalidates a capture
+// in progress.)
+cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, Graph& g) {
+  const Shape& shape = g.shape;
+  cudaError_t e = cudaGraphCreate(&g.graph, 0);
   if (e != cudaSuccess) return e;
+  cudaGraph_t graph = g.graph;
   using Nodes = std::vector<cudaGraphNode_t>;
   auto clear = [&](void* p, size_t words) {
     cudaGraphNode_t node = nullptr;
@@ -684,63 +683,100 @@ cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, cons
   // first: its walks end one by one and brute force fills in behind them (the
   // other way round the batch ends on the walks).
   for (int c = 0; c < kClasses; c++) {
-    if (!((shape.classes >> c) & 1u)) continue;
-    const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
+    if (!((g.classes >> c) & 1u)) continue;
+    const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query);
     const int fit = class_occupancy(c, smem);
     const unsigned blocks =
         (unsigned)((shape.per_sm_cap > 0 ? std::min(shape.per_sm_cap, fit) : fit) * sm_count_);
-    const int words = class_warp_words(c, shape.bh_stack, shape.bh_query, shape.sbh_root);
+    const int words = class_warp_words(c, shape.bh_stack, shape.bh_query);
     if (c < kClassBf)
-      kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items, d_trees,
-             (const int*)d_order_, d_status, words, shape.bh_stack);
+      g.node[c] = kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items,
+                         d_trees, (const int*)d_order_, d_status, words, shape.bh_stack);
     else
-      kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items, d_trees, words,
-             d_partial_, d_counters_);
+      g.node[c] = kernel(class_kernel(c), blocks, kEvalThreads, smem, ordered, d_header_, items,
+                         d_trees, words, d_partial_, d_counters_);
   }
-  if (e == cudaSuccess) e = cudaGraphInstantiate(out, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) *out = nullptr;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+  g.enabled = g.classes;
   return e;
+}
+
+cudaError_t BatchEngine::find_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
+                                    unsigned classes, cudaGraphExec_t* out) {
+  // Without Barnes-Hut in the batch any graph of the other parameters serves.
+  const bool bh = (classes >> kClassBh) & 1u;
+  size_t at = 0;
+  for (; at < graphs_.size(); at++) {
+    Shape s = graphs_[at].shape;
+    if (!bh || s.bh_stack == 0) {
+      s.bh_stack = shape.bh_stack;
+      s.bh_query = shape.bh_query;
+    }
+    if (s == shape) break;
+  }
+  if (at == graphs_.size() || (classes & ~graphs_[at].classes)) {
+    Graph g;
+    g.shape = shape;
+    g.classes = classes;
+    if (at < graphs_.size()) {
+      // A second set of classes: now all of them (Barnes-Hut once its stack is known), so
+      // that no later set costs a build (0.1 ms a node; switching nodes a few us).
+      if (!bh) {
+        g.shape.bh_stack = graphs_[at].shape.bh_stack;
+        g.shape.bh_query = graphs_[at].shape.bh_query;
+      }
+      g.classes = (1u << kClasses) - 1u;
+      if (g.shape.bh_stack == 0) g.classes &= ~(1u << kClassBh);
+      release(graphs_[at]);
+      graphs_.erase(graphs_.begin() + at);
+    } else if (graphs_.size() >= 32) {  // shapes are few; never let them pile up
+      for (Graph& old : graphs_) release(old);
+      graphs_.clear();
+    }
+    cudaError_t e = build_graph(d_trees, d_status, g);
+    if (e != cudaSuccess) {
+      release(g);
+      return e;
+    }
+    at = graphs_.size();
+    graphs_.push_back(g);
+  }
+  Graph& g = graphs_[at];
+  for (int c = 0; c < kClasses; c++) {
+    const unsigned bit = 1u << c;
+    if (((classes ^ g.enabled) & bit) == 0) continue;
+    cudaError_t e = cudaGraphNodeSetEnabled(g.exec, g.node[c], (classes & bit) != 0);
+    if (e != cudaSuccess) return e;
+    g.enabled ^= bit;
+  }
+  *out = g.exec;
+  return cudaSuccess;
 }
 
 cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTree* d_trees,
                                 int* d_status, cudaStream_t stream, const Tuning& tuning) {
   if (!dev_ || !h_stage_) return cudaErrorMemoryAllocation;
   if (captured_trees_ != d_trees || captured_status_ != d_status) {
-    for (Graph& g : graphs_)
-      if (g.exec) cudaGraphExecDestroy(g.exec);
+    for (Graph& g : graphs_) release(g);
     graphs_.clear();
     captured_trees_ = d_trees;
     captured_status_ = d_status;
   }
-  int need_depth = 0, need_root = 0;
+  int need_depth = -1;
+  unsigned classes = 0;
+  Shape shape;
+  shape.per_sm_cap = std::max(0, tuning.blocks_per_sm);
   for (const BatchItem& it : items) {
     const int c = batch_class(it.method, it.dim, it.kernel);
     if (c == kClassBh) need_depth = std::max(need_depth, it.depth);
-    if (c == kClassSbh) need_root = std::max(need_root, it.root_children);
-  }
-  Shape shape;
-  shape.per_sm_cap = std::max(0, tuning.blocks_per_sm);
-  shape.bh_stack = round_stack(need_depth + 2, lim_);
-  shape.sbh_root = round_root(need_root, lim_);
-  for (const BatchItem& it : items) {
     shape.bh_query = shape.bh_query || it.per_query;
     shape.sorted = shape.sorted || it.sort_bits > 0;
-    shape.classes |= 1u << batch_class(it.method, it.dim, it.kernel);
+    classes |= 1u << c;
   }
+  if (need_depth >= 0) shape.bh_stack = round_stack(need_depth + 2, lim_);
   cudaGraphExec_t exec = nullptr;
-  for (const Graph& g : graphs_)
-    if (g.shape == shape) exec = g.exec;
-  if (!exec) {
-    if (graphs_.size() >= 32) {  // shapes are few; never let them pile up
-      for (Graph& g : graphs_)
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-      graphs_.clear();
-    }
-    cudaError_t e = build_graph(d_trees, d_status, shape, &exec);
-    if (e != cudaSuccess) return e;
-    graphs_.push_back(Graph{shape, exec});
-  }
+  cudaError_t e = find_graph(d_trees, d_status, shape, classes, &exec);
+  if (e != cudaSuccess) return e;
   BatchHeader h = {};
   long long split_tiles = 0;
   h.n_items = (int)items.size();
@@ -763,8 +799,8 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
   std::memcpy(st, &h, sizeof(h));
   const size_t o_items = align256(sizeof(BatchHeader));
   if (!items.empty()) std::memcpy(st + o_items, items.data(), sizeof(BatchItem) * items.size());
-  cudaError_t e = cudaMemcpyAsync(d_header_, st, o_items + sizeof(BatchItem) * items.size(),
-                                  cudaMemcpyHostToDevice, stream);
+  e = cudaMemcpyAsync(d_header_, st, o_items + sizeof(BatchItem) * items.size(),
+                      cudaMemcpyHostToDevice, stream);
   // The counters of this batch's split tiles, on the stream that runs it: nothing
   // else orders a clearing before a batch (the default stream's work does not come
   // before a non-blocking stream's).

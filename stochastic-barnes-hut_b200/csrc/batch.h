@@ -122,25 +122,33 @@ class BatchEngine {
   }
 
  private:
-  // What a pipeline's graph is specialised for.
+  // What a pipeline's graph is specialised for.  The classes a batch has are not
+  // part of it: a graph has a kernel node for each class, or for those of its first
+  // batch while there is no other set, and a batch enables those of its own.
   struct Shape {
     int per_sm_cap = 0;  // the tuning's CTAs-per-SM cap (0: none)
-    int bh_stack = 0;    // Barnes-Hut stack entries per warp
-    bool bh_query = false;  // whether the scratch holds bh_query_task's
-    int sbh_root = 0;    // widest sampler root the scratch holds
-    unsigned classes = 0;  // bit c: the batch has requests of class c
     bool sorted = false;  // whether some request's queries are ordered
+    int bh_stack = 0;    // Barnes-Hut stack entries per warp (0: no Barnes-Hut class)
+    bool bh_query = false;  // whether the scratch holds bh_query_task's
     bool operator==(const Shape& o) const {
-      return per_sm_cap == o.per_sm_cap && bh_stack == o.bh_stack && bh_query == o.bh_query &&
-             sbh_root == o.sbh_root && classes == o.classes && sorted == o.sorted;
+      return per_sm_cap == o.per_sm_cap && sorted == o.sorted && bh_stack == o.bh_stack &&
+             bh_query == o.bh_query;
     }
   };
   struct Graph {
     Shape shape;
+    unsigned classes = 0;  // bit c: the graph has class c's kernel node, node[c] ...
+    unsigned enabled = 0;  // ... and runs it
+    cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    cudaGraphNode_t node[kClasses] = {};
   };
-  cudaError_t build_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
-                          cudaGraphExec_t* out);
+  cudaError_t build_graph(const DevTree* d_trees, int* d_status, Graph& g);
+  // The graph for a batch of `classes` (built or extended if need be), with exactly
+  // those enabled.
+  cudaError_t find_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
+                         unsigned classes, cudaGraphExec_t* out);
+  static void release(Graph& g);
 
   Limits lim_;
   int sm_count_;

@@ -1,0 +1,54 @@
+"""Batches of ever new mixes of request kinds on one engine: the pipeline is not built anew for a
+mix whose kinds were all seen before, and the results are those of each kind on its own."""
+import random
+import time
+
+import numpy as np
+import pytest
+
+import sbh_capi as C
+import sbh_workloads as W
+from helpers import bits_equal
+
+pytestmark = pytest.mark.gpu
+NQ = 70
+
+
+def test_new_mixes():
+    torch = pytest.importorskip("torch")
+    trees, queries = {}, {}
+    for dim in (2, 3):
+        pts, nrm, m = W.gaussian_mixture(3000, seed=2, dim=dim)
+        lo, hi = W.padded_box(pts)
+        trees[dim] = C.GpuTree.build(pts, nrm, m, lo, hi, alpha=9.0)
+        q = W.uniform_queries(NQ, seed=4, dim=dim)
+        queries[dim] = torch.from_numpy(np.ascontiguousarray(q.T)).cuda()
+    kinds = [(d, C.BRUTE_FORCE, k) for d in (2, 3)
+             for k in (C.GRAVITY, C.WINDING_NUMBER, C.SMOOTH_DIST, C.PLUMMER)]
+    kinds += [(3, C.BARNES_HUT, C.GRAVITY), (2, C.STOCHASTIC, C.PLUMMER)]
+    stream = torch.cuda.Stream()
+
+    def call(mix):
+        outs = [torch.full((NQ,), -7.0, device="cuda") for _ in mix]
+        items = [(trees[d], C.params(method=meth, kernel=k, seed=3), queries[d].data_ptr(), NQ,
+                  out.data_ptr(), 0, 0) for (d, meth, k), out in zip(mix, outs)]
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        C.eval_batch(items, stream=stream.cuda_stream)
+        t1 = time.perf_counter()
+        torch.cuda.synchronize()
+        return [o.cpu().numpy() for o in outs], t1 - t0
+
+    call(kinds)  # an engine with room for all, every kernel loaded
+    alone = {kind: call([kind])[0][0] for kind in kinds}
+    rng = random.Random(1)
+    first, again = [], []
+    for i in range(40):  # more mixes than an engine keeps pipelines
+        mix = rng.sample(kinds, rng.randint(2, len(kinds)))
+        got, t = call(mix)
+        first.append(t)
+        for kind, v in zip(mix, got):
+            assert bits_equal(v, alone[kind]), kind
+        again.append(min(call(mix)[1] for _ in range(3)))
+    # building a pipeline of two to ten kernels takes 0.2 to 2 ms, a call 0.03 to 0.06
+    assert np.median(first) <= 2 * np.median(again) + 50e-6
