@@ -91,21 +91,14 @@ __global__ void __launch_bounds__(AD_THREADS, 7)
 template <class A>
 struct CompSum;
 
-__device__ __forceinline__ void two_sum_into(float& hi, float& lo, float s) {
-  const float t = hi + s;
-  const float bp = t - hi;
-  lo += (hi - (t - bp)) + (s - bp);
-  hi = t;
-}
-
 template <int DIM, int K>
 struct CompSum<SumGrad<DIM, K>> {
   GradValue hi{0.f, 0.f, 0.f, 0.f}, lo{0.f, 0.f, 0.f, 0.f};
   __device__ __forceinline__ void add(const GradValue& p) {
-    two_sum_into(hi.v, lo.v, p.v);
-    two_sum_into(hi.gx, lo.gx, p.gx);
-    two_sum_into(hi.gy, lo.gy, p.gy);
-    two_sum_into(hi.gz, lo.gz, p.gz);
+    two_sum_add(hi.v, lo.v, p.v);
+    two_sum_add(hi.gx, lo.gx, p.gx);
+    two_sum_add(hi.gy, lo.gy, p.gy);
+    two_sum_add(hi.gz, lo.gz, p.gz);
   }
   __device__ __forceinline__ void merge(const CompSum& b) {
     add(b.hi);
@@ -130,10 +123,10 @@ struct CompSum<SumLse<DIM>> {
       const float f = expf(p.m - hi.m);
       p = LseValue{hi.m, p.s * f, p.gx * f, p.gy * f, p.gz * f};
     }
-    two_sum_into(hi.s, lo.s, p.s);
-    two_sum_into(hi.gx, lo.gx, p.gx);
-    two_sum_into(hi.gy, lo.gy, p.gy);
-    two_sum_into(hi.gz, lo.gz, p.gz);
+    two_sum_add(hi.s, lo.s, p.s);
+    two_sum_add(hi.gx, lo.gx, p.gx);
+    two_sum_add(hi.gy, lo.gy, p.gy);
+    two_sum_add(hi.gz, lo.gz, p.gz);
   }
   __device__ __forceinline__ void merge(const CompSum& b) {
     add(b.hi);
@@ -458,13 +451,6 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
 }
 
 }  // namespace
-
-size_t gradient_smem_bytes(const DevTree& t, int kernel) {
-  (void)t;
-  const size_t words = kernel == kSmoothDist ? sbh_warp_words<LseValue>()
-                                             : sbh_warp_words<GradValue>();
-  return (size_t)AD_WARPS * words * sizeof(float);
-}
 
 cudaError_t launch_gradient(const DevTree& t, int method, int kernel, const float* q, long long nq,
                             const int* order, float beta, int samples, unsigned long long seed,

@@ -568,7 +568,6 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
     if (it.tree < 0 || it.tree >= (int)host_trees.size()) return "request names an unknown tree";
     const DevTree& t = host_trees[it.tree];
     if (t.depth + 2 > lim_.max_tree_depth + 2) return "tree deeper than the engine supports";
-    if (t.root_children > lim_.max_root_children) return "tree root wider than the engine supports";
     it.per_query = it.method == 1 && (all_per_query || it.nq <= kBhUnorderedQueries);
     // vote and the sampler keep the caller's order, and so do few walks
     const bool sorted = it.method == 1 && !(it.per_query && it.nq <= kBhUnorderedQueries);
@@ -576,7 +575,6 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
         (sorted && it.sort_bits >= 0) ? sort_bits_for(it.nq, t.dim, tuning.bucket_queries) : 0;
     it.dim = t.dim;
     it.depth = t.depth;
-    it.root_children = t.root_children;
     it.sort_base = sort_base;
     it.bucket_base = bucket_base;
     it.buckets = it.sort_bits > 0 ? (1LL << (t.dim * it.sort_bits)) : 1;

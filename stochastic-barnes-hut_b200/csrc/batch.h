@@ -25,8 +25,7 @@ struct BatchItem {
   float beta;                // Barnes-Hut
   int sort_bits;             // Morton bits per axis of the query bucketing (0: keep order)
   int unit_queries;          // queries per work unit
-  int depth;                 // the tree's depth and root width (size the launch's
-  int root_children;         // shared memory; the kernels read the tree record's)
+  int depth;                 // the tree's depth (sizes the launch's shared memory)
   KParams kp;
   unsigned long long seed;   // stochastic method
   const float* q;            // device SoA [dim][nq]
@@ -92,7 +91,6 @@ class BatchEngine {
     int max_items = 4096;
     long long max_queries = 1 << 20;   // sorted positions (sum of request sizes)
     int max_tree_depth = 128;          // deepest tree the engine will see
-    int max_root_children = 512;       // widest root the engine will see
   };
 
   // Creates the engine on the current device; `trees` is a device table of

@@ -78,12 +78,9 @@ cudaError_t run_eval(sbh_gpu_tree* tree, const sbh_params* p, const float* d_q, 
 }
 
 // Extra checks of the gradient entry points.
-int check_grad_params(const sbh_gpu_tree* tree, const sbh_params* p) {
+int check_grad_params(const sbh_params* p) {
   if (p->kernel == SBH_KERNEL_WINDING_NUMBER)
     return sbh::fail(SBH_ERR_UNSUPPORTED, "gradients of gravity, Plummer and smooth distance only");
-  if (p->method == SBH_METHOD_STOCHASTIC &&
-      sbh::gradient_smem_bytes(tree->dev, p->kernel) > 227 * 1024)
-    return sbh::fail(SBH_ERR_UNSUPPORTED, "root too wide for the stochastic gradient kernel");
   return SBH_OK;
 }
 
@@ -92,7 +89,7 @@ int blocking_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* que
                   float* results, float* grads, int32_t* contribs, float* kernel_ms,
                   void* stream_ptr, bool grad) {
   int st = sbh::check_eval_params(tree, params, nq);
-  if (st == SBH_OK && grad) st = check_grad_params(tree, params);
+  if (st == SBH_OK && grad) st = check_grad_params(params);
   if (st != SBH_OK) return st;
   if (nq > 0 && (!queries || !results))
     return sbh::fail(SBH_ERR_INVALID_ARGUMENT, "queries and results must be non-null");
@@ -167,7 +164,7 @@ int device_eval(sbh_gpu_tree* tree, const sbh_params* params, const float* d_que
                 float* d_results, float* d_grads, int32_t* d_contribs, void* stream_ptr,
                 bool grad) {
   int st = sbh::check_eval_params(tree, params, nq);
-  if (st == SBH_OK && grad) st = check_grad_params(tree, params);
+  if (st == SBH_OK && grad) st = check_grad_params(params);
   if (st != SBH_OK) return st;
   if (nq == 0) return sbh::ok();
   if (!d_queries || !d_results)

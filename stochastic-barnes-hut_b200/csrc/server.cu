@@ -64,18 +64,13 @@ BatchEngine::Limits limits_for(const std::vector<DevTree>& trees, int max_items,
   lim.max_items = std::max(1, max_items);
   lim.max_queries = std::max(1LL, max_queries);
   lim.max_tree_depth = 1;
-  lim.max_root_children = 1;
-  for (const DevTree& t : trees) {
-    lim.max_tree_depth = std::max(lim.max_tree_depth, t.depth);
-    lim.max_root_children = std::max(lim.max_root_children, t.root_children);
-  }
+  for (const DevTree& t : trees) lim.max_tree_depth = std::max(lim.max_tree_depth, t.depth);
   return lim;
 }
 
 bool covers(const BatchEngine::Limits& have, const BatchEngine::Limits& need) {
   return have.max_items >= need.max_items && have.max_queries >= need.max_queries &&
-         have.max_tree_depth >= need.max_tree_depth &&
-         have.max_root_children >= need.max_root_children;
+         have.max_tree_depth >= need.max_tree_depth;
 }
 
 // ------------------------------------------------------------ sbh_eval_batch
@@ -264,7 +259,6 @@ int enqueue_batch(BatchContext& ctx, const sbh_batch_item* items, int n_items,
       grow.max_items = std::max(grow.max_items, o.max_items);
       grow.max_queries = std::max(grow.max_queries, o.max_queries);
       grow.max_tree_depth = std::max(grow.max_tree_depth, o.max_tree_depth);
-      grow.max_root_children = std::max(grow.max_root_children, o.max_root_children);
     }
     grow.max_items = std::max(grow.max_items * 2, 256);
     grow.max_queries = std::max(grow.max_queries * 2, 1LL << 16);
