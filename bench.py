@@ -465,7 +465,8 @@ def run_ours(args, wl):
             definition = (f"{bpe} B per kernel evaluation (node or point record) + 16 B per "
                           "query (SURVEY 8(d) per-unit figure; the opening tests' 32 B reads are "
                           "not counted)")
-            # a warp per query in calls of up to 2,048 queries per SM, a lane per query beyond
+            # a warp per query up to a line of queries per SM (2,048 for trees of these sizes),
+            # a lane per query beyond
             kernel_name = "barnes_hut_query_kernel" if nq <= 2048 * 148 else "barnes_hut_kernel"
         roofline = {
             "bound": "issue", "kernel": kernel_name,

@@ -405,7 +405,7 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
     const SplitShape shape = split_shape(nq, t.n, Acc::Q, Acc::kMinCtas, sm_count);
     return launch_split<Acc, DIM>(t, q, nq, kp, out, grads, contribs, stream, shape);
   }
-  if (method == SBH_METHOD_BARNES_HUT && bh_query_per_warp(nq, sm_count)) {
+  if (method == SBH_METHOD_BARNES_HUT && bh_query_per_warp(nq, t, sm_count)) {
     const size_t smem = AD_WARPS * bh_query_smem(t.depth);
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(bh_grad_query_kernel<DIM, K, A>,

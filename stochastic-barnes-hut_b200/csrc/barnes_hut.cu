@@ -131,7 +131,7 @@ cudaError_t launch_barnes_hut(const DevTree& t, int kernel, bool vote, const flo
   if (nq <= 0) return cudaSuccess;
 #define SBH_BH_CASE(D, K)                                                                      \
   if (t.dim == D && kernel == K)                                                               \
-    return !vote && !stage_leaves && bh_query_per_warp(nq, sm_count)                           \
+    return !vote && !stage_leaves && bh_query_per_warp(nq, t, sm_count)                           \
                ? launch_bh_query<D, K>(t, q, nq, order, beta, kp, out, contribs, status, stream) \
            : vote         ? launch_bh<D, K, true, false>(t, q, nq, order, beta, kp, out,       \
                                                          contribs, status, stream, sm_count)   \

@@ -548,12 +548,19 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
       bf_work += (double)((it.nq + kBfTileQueries - 1) / kBfTileQueries) *
                  (double)host_trees[it.tree].n;
   }
-  // Barnes-Hut walks: a warp per query under the same rule as a single call,
-  // here by the batch's queries, and in larger batches for requests of up to
-  // kBhUnorderedQueries, whose neighbours share too little of a walk (40 requests
-  // of 1 to 100,000 queries, theta 0.2: 22.9 ms a lane per query throughout, 12.1
-  // with this); units of a few queries where there are many.
-  const bool all_per_query = bh_query_per_warp(walked, sm_count_);
+  // Barnes-Hut walks: a warp per query under the same rule as a single call, here by
+  // the batch's queries, and in larger batches for requests of up to
+  // kBhUnorderedQueries whose queries lie too far apart for neighbours to share a walk:
+  // a twelfth of the tree's nodes at most in 3D, a hundredth in 2D (us, lane / warp per
+  // query, theta 0.5: 100 requests of 10,000 queries, 3D Gaussian mixtures of 10,000
+  // points 1,955 / 2,515, of 100,000 5,085 / 3,046, 2D circles of 1,000 469 / 2,181, of
+  // 100,000 834 / 2,204; 1,000 of 1,000, 3D of 1,000 1,743 / 2,828, 2D of 100,000 4,328 /
+  // 3,464); units of a few queries where there are many.
+  auto per_query = [&](const BatchItem& it, const DevTree& t) {
+    return it.method == 1 &&
+           (bh_query_per_warp(walked, t, sm_count_) ||
+            (it.nq <= kBhUnorderedQueries && it.nq * (t.dim == 3 ? 12 : 100) <= t.nn));
+  };
   int walk_unit = 1;
   while (walk_unit < 8 && walked > 64LL * walk_unit * sm_count_) walk_unit *= 2;
   // Brute force: a tile's sum over all sources is one unit while that is at most
@@ -568,7 +575,7 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
     if (it.tree < 0 || it.tree >= (int)host_trees.size()) return "request names an unknown tree";
     const DevTree& t = host_trees[it.tree];
     if (t.depth + 2 > lim_.max_tree_depth + 2) return "tree deeper than the engine supports";
-    it.per_query = it.method == 1 && (all_per_query || it.nq <= kBhUnorderedQueries);
+    it.per_query = per_query(it, t);
     // vote and the sampler keep the caller's order, and so do few walks
     const bool sorted = it.method == 1 && !(it.per_query && it.nq <= kBhUnorderedQueries);
     it.sort_bits =

@@ -34,7 +34,7 @@ bool wants_sort(const sbh_params* p) {
 bool needs_order(const sbh_gpu_tree* tree, const sbh_params* p, int64_t nq) {
   if (!wants_sort(p) || p->method != SBH_METHOD_BARNES_HUT) return false;
   return (p->flags & SBH_FLAG_STAGE_LEAVES) || nq > sbh::kBhUnorderedQueries ||
-         !sbh::bh_query_per_warp(nq, tree->sm_count);
+         !sbh::bh_query_per_warp(nq, tree->dev, tree->sm_count);
 }
 
 // Enqueues one evaluation.  With `grad` the adjoint kernels run instead (values

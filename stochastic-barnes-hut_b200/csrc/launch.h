@@ -3,6 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "device_common.cuh"
 
 namespace sbh {
@@ -10,21 +13,28 @@ namespace sbh {
 cudaError_t launch_brute_force(const DevTree& t, int kernel, const float* q, long long nq,
                                const KParams& kp, float* out, cudaStream_t stream, int sm_count);
 
-// Barnes-Hut calls of up to 2,048 queries per SM run a warp per query
-// (bh_query_task), larger ones a lane per query (bh_warp_task).  A lane per query
-// does a node test in fewer instructions, but a call lasts at least as long as
-// its longest walk, one node after the other.  Measured on B200 (us, lane / warp
-// per query, theta 0.5): 1M-point torus, branching 64: 1,000 queries 2,910 / 170,
-// 65,536 4,206 / 1,032, 200,000 5,207 / 2,833, 300,000 5,252 / 4,194, 500,000 6,085 /
-// 6,950; 10,000-point Gaussian mixture, branching 8: 490 / 54, 603 / 236, 725 / 545,
-// 689 / 799, 751 / 1,290; 65,536 points, leaf 8: 1,414 / 282, 2,009 / 576, 2,298 /
-// 1,164, 2,370 / 1,635, 2,299 / 2,603.
-inline bool bh_query_per_warp(long long nq, int sm_count) { return nq <= 2048LL * sm_count; }
 // Without neighbours sharing a warp the query order only helps the L1 cache; up
 // to this many queries that is worth less than the ordering's seven launches
-// (16,000 queries on the same trees: 379 -> 384 and 122 -> 94 us without it;
-// 65,536: 1,015 -> 1,105 and 227 -> 220).
+// (1M-point torus and 10,000-point Gaussian mixture: 16,000 queries 379 -> 384 and
+// 122 -> 94 us without it; 65,536 1,015 -> 1,105 and 227 -> 220).
 constexpr long long kBhUnorderedQueries = 16384;
+
+// Barnes-Hut calls run a warp per query (bh_query_task) up to a number of queries, a
+// lane per query (bh_warp_task) beyond.  A lane per query does a node test in fewer
+// instructions, but a call lasts at least as long as its longest walk, one node after
+// the other, and that grows with the tree.  Measured on B200 (us, lane / warp per query,
+// theta 0.5): circle in 2D, 1,000 points: 20,000 queries 78 / 70, 40,000 104 / 101,
+// 300,000 104 / 523; 150,000 points: 40,000 248 / 111, 150,000 363 / 284, 300,000 469 /
+// 532; torus, 1,000 points: 40,000 431 / 197, 80,000 462 / 350, 300,000 429 / 1,185;
+// 40,000 points: 150,000 1,498 / 1,004, 300,000 1,503 / 1,954; 1M points: 300,000 3,406 /
+// 2,156; 500,000 (branching 64) 6,085 / 6,950.  Over 1,872 calls (2D and 3D, 100 to 1M
+// points, leaves of 1 and 8, theta 0.2 to 0.8, gradients) this line costs 2% over the
+// better of the two; 2,048 queries per SM whatever the tree cost 30%, and 5 times the
+// lane walk's time on small trees.
+inline bool bh_query_per_warp(long long nq, const DevTree& t, int sm_count) {
+  const double per_sm = (t.dim == 3 ? 15.0 : 7.0) * std::sqrt((double)t.nn);
+  return nq <= kBhUnorderedQueries || (double)nq <= std::min(per_sm, 2048.0) * sm_count;
+}
 
 // stage_leaves: accepted multi-point leaves are copied to shared memory by bulk
 // asynchronous copies (SBH_FLAG_STAGE_LEAVES; not with vote).
