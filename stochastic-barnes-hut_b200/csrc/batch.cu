@@ -504,7 +504,8 @@ BatchEngine::BatchEngine(const Limits& lim, int sm_count) : lim_(lim), sm_count_
 }
 
 BatchEngine::~BatchEngine() {
-  for (Graph& g : graphs_) release(g);
+  release_all(graphs_);
+  release_all(any_);
   if (h_stage_) cudaFreeHost(h_stage_);
   if (dev_) cudaFree(dev_);
 }
@@ -620,11 +621,15 @@ std::string BatchEngine::plan(std::vector<BatchItem>& items,
 void BatchEngine::release(Graph& g) {
   if (g.exec) cudaGraphExecDestroy(g.exec);
   if (g.graph) cudaGraphDestroy(g.graph);
-  g.exec = nullptr;
-  g.graph = nullptr;
+  g = Graph();
 }
 
-// Builds the pipeline's graph of g's shape and classes node by node.  (Capturing it
+void BatchEngine::release_all(std::vector<Graph>& graphs) {
+  for (Graph& g : graphs) release(g);
+  graphs.clear();
+}
+
+// Builds the pipeline's graph of g's shape node by node.  (Capturing it
 // from streams cost a stream and an event per branch, 0.5 ms each, and any other
 // thread's device synchronisation -- a tree being destroyed -- invalidates a capture
 // in progress.)
@@ -688,7 +693,7 @@ cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, Grap
   // first: its walks end one by one and brute force fills in behind them (the
   // other way round the batch ends on the walks).
   for (int c = 0; c < kClasses; c++) {
-    if (!((g.classes >> c) & 1u)) continue;
+    if (!((shape.classes >> c) & 1u)) continue;
     const size_t smem = class_smem(c, shape.bh_stack, shape.bh_query);
     const int fit = class_occupancy(c, smem);
     const unsigned blocks =
@@ -702,55 +707,70 @@ cudaError_t BatchEngine::build_graph(const DevTree* d_trees, int* d_status, Grap
                          d_trees, words, d_partial_, d_counters_);
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
-  g.enabled = g.classes;
+  g.enabled = shape.classes;
+  if (e != cudaSuccess) release(g);
   return e;
 }
 
+// A graph of the batch's own classes is the fastest to launch (with nodes switched from
+// batch to batch the serving stream at twice the plain capacity fell from 22.3 to 20.6 M
+// queries/s), and building one takes 0.1 to 2 ms, 0.1 a kernel.  So the first shapes
+// get their own, and later ones when they come a second time; until then a graph of
+// all classes serves them with the others' nodes switched off (45 us more).
 cudaError_t BatchEngine::find_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
-                                    unsigned classes, cudaGraphExec_t* out) {
-  // Without Barnes-Hut in the batch any graph of the other parameters serves.
-  const bool bh = (classes >> kClassBh) & 1u;
-  size_t at = 0;
-  for (; at < graphs_.size(); at++) {
-    Shape s = graphs_[at].shape;
-    if (!bh || s.bh_stack == 0) {
-      s.bh_stack = shape.bh_stack;
-      s.bh_query = shape.bh_query;
-    }
-    if (s == shape) break;
+                                    cudaGraphExec_t* out) {
+  constexpr size_t kFirst = 8, kMost = 32;
+  for (size_t i = 0; i < graphs_.size(); i++) {
+    if (!(graphs_[i].shape == shape)) continue;
+    std::rotate(graphs_.begin() + i, graphs_.begin() + i + 1, graphs_.end());
+    *out = graphs_.back().exec;
+    return cudaSuccess;
   }
-  if (at == graphs_.size() || (classes & ~graphs_[at].classes)) {
+  const auto again = std::find(seen_.begin(), seen_.end(), shape);
+  if (graphs_.size() < kFirst || again != seen_.end()) {
     Graph g;
     g.shape = shape;
-    g.classes = classes;
-    if (at < graphs_.size()) {
-      // A second set of classes: now all of them (Barnes-Hut once its stack is known), so
-      // that no later set costs a build (0.1 ms a node; switching nodes a few us).
-      if (!bh) {
-        g.shape.bh_stack = graphs_[at].shape.bh_stack;
-        g.shape.bh_query = graphs_[at].shape.bh_query;
-      }
-      g.classes = (1u << kClasses) - 1u;
-      if (g.shape.bh_stack == 0) g.classes &= ~(1u << kClassBh);
-      release(graphs_[at]);
-      graphs_.erase(graphs_.begin() + at);
-    } else if (graphs_.size() >= 32) {  // shapes are few; never let them pile up
-      for (Graph& old : graphs_) release(old);
-      graphs_.clear();
-    }
     cudaError_t e = build_graph(d_trees, d_status, g);
-    if (e != cudaSuccess) {
-      release(g);
-      return e;
+    if (e != cudaSuccess) return e;
+    if (again != seen_.end()) seen_.erase(again);
+    if (graphs_.size() >= kMost) {  // the one not used for longest
+      release(graphs_.front());
+      graphs_.erase(graphs_.begin());
     }
-    at = graphs_.size();
     graphs_.push_back(g);
+    *out = g.exec;
+    return cudaSuccess;
   }
-  Graph& g = graphs_[at];
+  if (seen_.size() >= 64) seen_.erase(seen_.begin());
+  seen_.push_back(shape);
+  // One of all classes serves the batch if their other parameters agree (Barnes-Hut's
+  // matter to a batch that has it, and not to a graph without it).
+  constexpr unsigned kBh = 1u << kClassBh, kAll = (1u << kClasses) - 1u;
+  size_t at = 0;
+  for (; at < any_.size(); at++) {
+    Shape s = any_[at].shape;
+    if (shape.bh_stack == 0) s.bh_stack = 0, s.bh_query = false;
+    s.classes = shape.classes;
+    if (s == shape) break;
+  }
+  if (at == any_.size()) {
+    Graph g;
+    g.shape = shape;
+    g.shape.classes = shape.bh_stack ? kAll : kAll & ~kBh;
+    cudaError_t e = build_graph(d_trees, d_status, g);
+    if (e != cudaSuccess) return e;
+    if (any_.size() >= 4) {
+      release(any_.front());
+      any_.erase(any_.begin());
+    }
+    any_.push_back(g);
+    at = any_.size() - 1;
+  }
+  Graph& g = any_[at];
   for (int c = 0; c < kClasses; c++) {
     const unsigned bit = 1u << c;
-    if (((classes ^ g.enabled) & bit) == 0) continue;
-    cudaError_t e = cudaGraphNodeSetEnabled(g.exec, g.node[c], (classes & bit) != 0);
+    if (((shape.classes ^ g.enabled) & bit) == 0) continue;
+    cudaError_t e = cudaGraphNodeSetEnabled(g.exec, g.node[c], (shape.classes & bit) != 0);
     if (e != cudaSuccess) return e;
     g.enabled ^= bit;
   }
@@ -762,13 +782,13 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
                                 int* d_status, cudaStream_t stream, const Tuning& tuning) {
   if (!dev_ || !h_stage_) return cudaErrorMemoryAllocation;
   if (captured_trees_ != d_trees || captured_status_ != d_status) {
-    for (Graph& g : graphs_) release(g);
-    graphs_.clear();
+    release_all(graphs_);
+    release_all(any_);
+    seen_.clear();
     captured_trees_ = d_trees;
     captured_status_ = d_status;
   }
   int need_depth = -1;
-  unsigned classes = 0;
   Shape shape;
   shape.per_sm_cap = std::max(0, tuning.blocks_per_sm);
   for (const BatchItem& it : items) {
@@ -776,11 +796,11 @@ cudaError_t BatchEngine::launch(const std::vector<BatchItem>& items, const DevTr
     if (c == kClassBh) need_depth = std::max(need_depth, it.depth);
     shape.bh_query = shape.bh_query || it.per_query;
     shape.sorted = shape.sorted || it.sort_bits > 0;
-    classes |= 1u << c;
+    shape.classes |= 1u << c;
   }
   if (need_depth >= 0) shape.bh_stack = round_stack(need_depth + 2, lim_);
   cudaGraphExec_t exec = nullptr;
-  cudaError_t e = find_graph(d_trees, d_status, shape, classes, &exec);
+  cudaError_t e = find_graph(d_trees, d_status, shape, &exec);
   if (e != cudaSuccess) return e;
   BatchHeader h = {};
   long long split_tiles = 0;

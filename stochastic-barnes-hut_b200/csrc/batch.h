@@ -120,33 +120,31 @@ class BatchEngine {
   }
 
  private:
-  // What a pipeline's graph is specialised for.  The classes a batch has are not
-  // part of it: a graph has a kernel node for each class, or for those of its first
-  // batch while there is no other set, and a batch enables those of its own.
+  // What a pipeline's graph is specialised for.
   struct Shape {
     int per_sm_cap = 0;  // the tuning's CTAs-per-SM cap (0: none)
     bool sorted = false;  // whether some request's queries are ordered
     int bh_stack = 0;    // Barnes-Hut stack entries per warp (0: no Barnes-Hut class)
     bool bh_query = false;  // whether the scratch holds bh_query_task's
+    unsigned classes = 0;  // bit c: a kernel node for class c
     bool operator==(const Shape& o) const {
       return per_sm_cap == o.per_sm_cap && sorted == o.sorted && bh_stack == o.bh_stack &&
-             bh_query == o.bh_query;
+             bh_query == o.bh_query && classes == o.classes;
     }
   };
   struct Graph {
     Shape shape;
-    unsigned classes = 0;  // bit c: the graph has class c's kernel node, node[c] ...
-    unsigned enabled = 0;  // ... and runs it
+    unsigned enabled = 0;  // bit c: class c's kernel node runs
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaGraphNode_t node[kClasses] = {};
   };
   cudaError_t build_graph(const DevTree* d_trees, int* d_status, Graph& g);
-  // The graph for a batch of `classes` (built or extended if need be), with exactly
-  // those enabled.
+  // The graph for a batch of this shape (built if need be).
   cudaError_t find_graph(const DevTree* d_trees, int* d_status, const Shape& shape,
-                         unsigned classes, cudaGraphExec_t* out);
+                         cudaGraphExec_t* out);
   static void release(Graph& g);
+  static void release_all(std::vector<Graph>& graphs);
 
   Limits lim_;
   int sm_count_;
@@ -165,8 +163,10 @@ class BatchEngine {
   unsigned* d_counters_ = nullptr;  // ... and how many of a tile's parts are done
   // pinned staging of header + items
   void* h_stage_ = nullptr;
-  // instantiated pipelines, one per launch shape
-  std::vector<Graph> graphs_;
+  // instantiated pipelines of recurring shapes, the last used at the end; some with all
+  // classes for shapes met once, and those shapes
+  std::vector<Graph> graphs_, any_;
+  std::vector<Shape> seen_;
   const DevTree* captured_trees_ = nullptr;
   int* captured_status_ = nullptr;
 };
