@@ -1237,8 +1237,9 @@ def run_serving(args):
         "setup_s": setup_s,
         "cpu_baseline": cpu,
         # per batch step: the graph's 9 kernels (query boxes, keys, three scan
-        # kernels, scatter, one persistent kernel per method class) plus 8 (sort
-        # and sampler) per stochastic request sent to its own launch
+        # kernels, scatter, and a persistent kernel each for Barnes-Hut and the
+        # smooth distance in 3D and 2D) plus one per stochastic request sent to its
+        # own launch
         "gpu_launches": args.steps * (9 + n_direct),
     }
 

@@ -13,7 +13,7 @@
 //     Plummer pair costs 3.5 FP32 issue slots plus one MUFU rsqrt.  Both pipes are
 //     loaded: 65,536 x 65,536 Plummer pairs take 1,180 us (0.79 of the MUFU bound;
 //     1,350 with a query per thread), smooth distance 1,980 (2,322), winding
-//     number 2,348 (2,519), gravity 2,105 (2,309).
+//     number 2,348 (2,519), gravity 1,919 (2,309).
 //   * Compensated accumulation in two levels: plain FP32 over 32 sources of a
 //     lane, then a Knuth two-sum into a (sum, error) pair -- the reference's Kahan
 //     loop (brute_force_gpu.h:52-60) at a fraction of its cost per pair.

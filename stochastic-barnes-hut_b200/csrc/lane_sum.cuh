@@ -84,7 +84,9 @@ template <int DIM, int K, int NP>
 struct PlainAcc {
   using Sum = PlainSum;
   static constexpr int Q = 2 * NP;
-  static constexpr int kMinCtas = NP == 4 ? 2 : K == kWindingNumber ? 3 : 4;  // no spills
+  // Spills (bytes loaded): 12 at most, but 40 and 112 in the 3D gravity and winding-number
+  // kernels of one pair.
+  static constexpr int kMinCtas = NP == 4 ? 2 : K == kWindingNumber ? 3 : 4;
   static constexpr bool kNormals = K == kWindingNumber;
   float2 nqx[NP], nqy[NP], nqz[NP], part[NP];
   float hi[Q], lo[Q];

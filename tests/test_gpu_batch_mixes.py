@@ -1,5 +1,5 @@
-"""Batches of ever new mixes of request kinds on one engine: the pipeline is not built anew for a
-mix whose kinds were all seen before, and the results are those of each kind on its own."""
+"""Batches of ever new mixes of request kinds on one engine: a mix met for the first time does not
+wait for a pipeline of its own, and the results are those of each kind on its own."""
 import random
 import time
 
