@@ -401,6 +401,9 @@ cudaError_t launch_policy(const DevTree& t, int method, const float* q, long lon
                           const KParams& kp, float* out, float* grads, int* contribs,
                           int* status, cudaStream_t stream, int sm_count) {
   if (method == SBH_METHOD_BRUTE_FORCE) {
+    if (lane_per_query(nq, t.n, sm_count, true))
+      return launch_lane_query<GradAcc<DIM, K, A, 1>, DIM>(t, q, nq, kp, out, grads, contribs,
+                                                           stream);
     using Acc = GradAcc<DIM, K, A, 2>;
     const SplitShape shape = split_shape(nq, t.n, Acc::Q, Acc::kMinCtas, sm_count);
     return launch_split<Acc, DIM>(t, q, nq, kp, out, grads, contribs, stream, shape);

@@ -33,6 +33,8 @@ cudaError_t launch_bf(const DevTree& t, const float* q, long long nq, const KPar
   // warp, smooth distance, 1M sources): 1 query 65 / 40, 40 67 / 52, 200 151 / 156.
   using Eight = PlainAcc<DIM, K, 4>;
   using Two = PlainAcc<DIM, K, 1>;
+  if (lane_per_query(nq, t.n, sm_count, false))
+    return launch_lane_query<Two, DIM>(t, q, nq, kp, out, nullptr, nullptr, stream);
   const SplitShape s8 = split_shape(nq, t.n, Eight::Q, Eight::kMinCtas, sm_count);
   const SplitShape s2 = split_shape(nq, t.n, Two::Q, Two::kMinCtas, sm_count);
   if (0.55 * s2.cost < s8.cost)

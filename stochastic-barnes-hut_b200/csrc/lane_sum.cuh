@@ -62,6 +62,29 @@ __device__ __forceinline__ void sum_range(Acc& acc, const float4* __restrict__ p
   acc.flush();
 }
 
+// Adds all of the n sources to a lane's state, the lane's own queries: every lane reads
+// the same sources.
+template <class Acc>
+__device__ __forceinline__ void sum_all(Acc& acc, const float4* __restrict__ pt_pm,
+                                        const float4* __restrict__ pt_nrm, long long n) {
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  long long base = 0;
+  int run = 0;
+  for (; base + kSplitGroup <= n; base += kSplitGroup) {
+    float4 s[kSplitGroup], nr[kSplitGroup];
+#pragma unroll
+    for (int i = 0; i < kSplitGroup; i++) {
+      s[i] = __ldg(pt_pm + base + i);
+      nr[i] = Acc::kNormals ? __ldg(pt_nrm + base + i) : none;
+    }
+    acc.group(s, nr);
+    if ((++run & (kSplitRun / kSplitGroup - 1)) == 0) acc.flush();
+  }
+  for (; base < n; base++)
+    acc.single(__ldg(pt_pm + base), Acc::kNormals ? __ldg(pt_nrm + base) : none);
+  acc.flush();
+}
+
 // The lanes' sums of one query, merged into lane 0's.
 template <class Sum>
 __device__ __forceinline__ Sum merge_lanes(Sum v) {

@@ -143,5 +143,47 @@ cudaError_t launch_split(const DevTree& t, const float* q, long long nq, const K
   return launch(8);
 }
 
+// Few sources and many queries: a lane per Acc::Q queries (sum_all), without the merging
+// of lanes' sums, which takes as long as 250 sources.
+template <class Acc, int DIM>
+__global__ void __launch_bounds__(kSplitThreads, Acc::kMinCtas)
+    lane_query_kernel(DevTree t, const float* __restrict__ qsoa, long long nq, KParams kp,
+                      float* __restrict__ out, float* __restrict__ grads,
+                      int* __restrict__ contribs) {
+  const long long q0 = ((long long)blockIdx.x * kSplitThreads + threadIdx.x) * Acc::Q;
+  if (q0 >= nq) return;
+  Acc acc;
+  acc.load(qsoa, nq, q0, kp);
+  sum_all(acc, t.pt_pm, t.pt_nrm, t.n);
+#pragma unroll
+  for (int j = 0; j < Acc::Q; j++) {
+    if (q0 + j >= nq) break;
+    Acc::store(out, grads, nq, q0 + j, acc.sum(j), kp);
+    if (contribs) contribs[q0 + j] = (int)t.n;
+  }
+}
+
+// Where that is the faster form: the call lasts as long as one lane's sum over all
+// sources, so the queries have to be many beside them, and beyond a few hundred sources
+// (some thousands for gradients, whose merging is longer) a warp's shared loads win.
+// Measured (us, split / lane per query, 3D): Plummer, 100 sources: 10,000 queries 7.5 /
+// 11.0, 30,000 13.0 / 10.9, 400,000 68 / 22; 300: 60,000 17 / 24, 100,000 25 / 24; 600:
+// 200,000 60 / 50; 1,000: 400,000 156 / 180, 2M 750 / 574; gradients of the smooth
+// distance, 100: 10,000 27 / 17, 400,000 554 / 50; 1,000: 60,000 151 / 121; 4,000: 200,000
+// 981 / 1,001, 400,000 1,931 / 1,471.
+inline bool lane_per_query(long long nq, long long n, int sm_count, bool gradients) {
+  if (gradients) return n <= 4096 && 2 * nq >= n * sm_count;
+  return n <= (nq >= 8192LL * sm_count ? 2048 : 768) && nq >= 2 * n * sm_count;
+}
+
+template <class Acc, int DIM>
+cudaError_t launch_lane_query(const DevTree& t, const float* q, long long nq, const KParams& kp,
+                              float* out, float* grads, int* contribs, cudaStream_t stream) {
+  const long long per_cta = (long long)kSplitThreads * Acc::Q;
+  lane_query_kernel<Acc, DIM><<<(unsigned)((nq + per_cta - 1) / per_cta), kSplitThreads, 0,
+                                stream>>>(t, q, nq, kp, out, grads, contribs);
+  return cudaGetLastError();
+}
+
 }  // namespace
 }  // namespace sbh
